@@ -89,9 +89,18 @@ struct Control {
 
 constexpr int VX_BLOCKS = 64;
 
+// What a step reads of a crash's control block: the resident step kernel keeps
+// a copy per block in shared memory, so the functions below take either.
+struct ControlView {
+    double t, end_time, dt_cfl, damping, dt_floor;
+    long long step, max_steps;
+    int done, mass_scale_now;
+};
+
 // The step's dt from the control block: dt_cfl clipped to the end time,
 // never below 1e-15 (src/solver.rs:300).
-__device__ __forceinline__ double step_dt(const Control* c) {
+template <class C>
+__device__ __forceinline__ double step_dt(const C* c) {
     double rem = c->end_time - c->t;
     double d = c->dt_cfl < rem ? c->dt_cfl : rem;
     return d > 1e-15 ? d : 1e-15;
@@ -100,7 +109,8 @@ __device__ __forceinline__ double step_dt(const Control* c) {
 // The dt of the step after the current one when no stable-dt check falls
 // between them: step_dt once the step's end has added this step's dt to t
 // (the same arithmetic, so it is the value the next step will use).
-__device__ __forceinline__ double next_step_dt(const Control* c) {
+template <class C>
+__device__ __forceinline__ double next_step_dt(const C* c) {
     const double t1 = c->t + step_dt(c);
     double rem = c->end_time - t1;
     double d = c->dt_cfl < rem ? c->dt_cfl : rem;
@@ -109,7 +119,8 @@ __device__ __forceinline__ double next_step_dt(const Control* c) {
 
 // Whether the current step is the crash's last by the step count or the end
 // time (the stop rules that need no reduction), as the step's end decides it.
-__device__ __forceinline__ bool last_step_by_count_or_time(const Control* c) {
+template <class C>
+__device__ __forceinline__ bool last_step_by_count_or_time(const C* c) {
     const double t1 = c->t + step_dt(c);
     return (c->max_steps > 0 && c->step + 1 >= c->max_steps) || !(t1 < c->end_time);
 }

@@ -459,13 +459,14 @@ struct crush_ctx {
     int *face_off_d = nullptr, *slave_off_d = nullptr, *tab_off_d = nullptr;
     long long *st_tab_off_d = nullptr, *ent_off_d = nullptr;
     uint32_t *faces_d = nullptr, *slaves_d = nullptr, *grid_faces_d = nullptr, *dyn_faces_d = nullptr, *gslaves_d = nullptr,
-             *stslaves_d = nullptr, *cnode_d = nullptr, *cnode_off_d = nullptr, *slave_cn_d = nullptr, *face_cn_d = nullptr,
+             *stslaves_d = nullptr, *node_cn = nullptr, *cnode_d = nullptr, *cnode_off_d = nullptr, *slave_cn_d = nullptr, *face_cn_d = nullptr,
              *st_off_d = nullptr, *vnodes_d = nullptr;
     double *scales_d = nullptr, *stiff_d = nullptr, *md_d = nullptr, *cell_d = nullptr, *st_box_d = nullptr;
     int *brute_d = nullptr, *counts_for_stop_d = nullptr, *crole_contact_d = nullptr, *crole_slave_d = nullptr, *face_contact_d = nullptr,
         *slave_contact_d = nullptr, *contact_slot_d = nullptr, *slot_contact_off_d = nullptr, *st_entries_d = nullptr, *vslot_d = nullptr,
         *vlocal_d = nullptr, *chunk_lo_d = nullptr, *chunk_hi_d = nullptr;
     uint8_t* is_static_d = nullptr;
+    BruteEntry* bents_d = nullptr;
     long long* voff_d = nullptr;
     double *sc_geo = nullptr, *sc_mat = nullptr, *sc_corner = nullptr;
     float4 *planes = nullptr, *state = nullptr;
@@ -536,6 +537,9 @@ struct crush_ctx {
     int n_sms = 148;
     int forces_schedule = CANDS[DEFAULT_CAND].forces;  // launch_forces schedule (0 persistent wave, 1 block per chunk, 2/3 wave on fewer SMs)
     bool fused_contact_side = false;      // a fused step's next contact forces on the side stream (else main, after the forces)
+    ResidentSync* res_sync = nullptr;     // device: the resident step kernel's barrier and outcome
+    int res_blocks = 0;                   // blocks of it the device holds at once (0: none)
+    bool res_used = false;                // it ran since the run began
     unsigned* forces_queue = nullptr;     // device: chunk queue of the persistent element-kernel waves
     // Slots added to an open run are set up on `setup`, beside the steps
     // issued last (the set-up writes only the new slots' ranges); the main
@@ -1468,6 +1472,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     // exhaustive contacts (no grid) get a block each; the rest are listed by entry
     std::vector<int> brute;
     std::vector<uint32_t> gslaves, stslaves;
+    std::vector<BruteEntry> bents;
     std::vector<uint8_t> is_brute(std::max(K, 1), 0);
     int brute_max = c->ca.brute_max_faces;
     for (int q = 0; q < K; ++q) {
@@ -1477,6 +1482,9 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
             brute.push_back(K0 + q);
             is_brute[q] = 1;
             brute_max = std::max(brute_max, face_off[q + 1] - face_off[q]);
+            for (int e = slave_off[q]; e < slave_off[q + 1]; ++e)
+                bents.push_back(BruteEntry{(uint32_t)e, slaves[e - base[0].slave], K0 + q, contact_slot[q], face_off[q],
+                                           face_off[q + 1] - face_off[q], {0, 0}});
         } else {
             for (int e = slave_off[q]; e < slave_off[q + 1]; ++e) (st_grid ? stslaves : gslaves).push_back((uint32_t)e);
         }
@@ -1673,6 +1681,10 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         TRY(c->alloc(&c->brute_d, KC));
         TRY(c->alloc(&c->gslaves_d, SC));
         TRY(c->alloc(&c->stslaves_d, SC));
+        TRY(c->alloc(&c->bents_d, SC));
+        TRY(c->alloc(&c->node_cn, NC));
+        TRY(c->alloc(&c->res_sync, 1));
+        c->res_blocks = resident_blocks(c->device, c->n_sms);
         TRY(c->alloc(&ca.grid_state, 2 * KC + 1));
         TRY(c->alloc(&ca.cells, FC));
         TRY(c->alloc(&ca.gather_work, CNC));
@@ -1720,6 +1732,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         ca.brute_contacts = c->brute_d;
         ca.grid_slaves = c->gslaves_d;
         ca.st_slaves = c->stslaves_d;
+        ca.brute_entries = c->bents_d;
         ca.counts_for_stop = c->counts_for_stop_d;
         ca.cnode = c->cnode_d;
         ca.cnode_off = c->cnode_off_d;
@@ -1823,6 +1836,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     TRY(put(c->brute_d + ca.n_brute, brute.data(), brute.size()));
     TRY(put(c->gslaves_d + ca.n_grid_slaves, gslaves.data(), gslaves.size()));
     TRY(put(c->stslaves_d + ca.n_st_slaves, stslaves.data(), stslaves.size()));
+    TRY(put(c->bents_d + ca.n_brute_entries, bents.data(), bents.size()));
     TRY(put(c->counts_for_stop_d + K0, counts_for_stop.data(), K));
     TRY(put(c->cnode_d + base[0].cnode, cnode.data(), cnode.size()));
     TRY(put(c->cnode_off_d + base[0].cnode, cnode_off.data(), cnode_off.size()));
@@ -1877,6 +1891,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     for (int q = 0; q < K; ++q) c->is_brute_h[K0 + q] = is_brute[q];
     c->grid_slaves_h.insert(c->grid_slaves_h.end(), gslaves.begin(), gslaves.end());
     c->st_slaves_h.insert(c->st_slaves_h.end(), stslaves.begin(), stslaves.end());
+    ca.n_brute_entries += (long long)bents.size();
     ca.n_contacts = c->n_contacts;
     ca.n_slots = c->n_slots;
     ca.n_buckets = tab_off[K];
@@ -1994,6 +2009,9 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     TRY(check_launch(c));
     launch_init_state(c->stream, H0, H0 + H, c->stride, c->state);
     TRY(check_launch(c));
+    CK(cudaMemsetAsync(c->node_cn + N0, 0xFF, sizeof(uint32_t) * N, c->stream));  // CN_NONE
+    launch_node_cn(c->stream, c->cnode_d, base[0].cnode, tot.cnode, c->node_cn);
+    TRY(check_launch(c, tot.cnode > base[0].cnode ? 1 : 0));
     // contact_dt over every listed node of the slot's contacts (src/solver.rs:217-223)
     std::vector<double> mass_h(N);
     int bad_h = 0;
@@ -2608,6 +2626,8 @@ Control initial_control(const Slot& sl) {
     return x;
 }
 
+bool resident(const crush_ctx* c);
+
 int run_begin(crush_ctx* c) {
     const long long N = c->n_nodes;
     drop_graphs(c);
@@ -2620,6 +2640,7 @@ int run_begin(crush_ctx* c) {
     CK(cudaMemsetAsync(c->fused_counter, 0, sizeof(unsigned), c->stream));
     c->prologue_done = false;
     c->contact_done = false;
+    c->res_used = false;
     if (c->n_contacts > 0) {
         CK(cudaMemsetAsync(c->ca.big_best, 0x7F, sizeof(int) * std::max<long long>(c->n_slaves, 1), c->stream));  // BIG_NONE
         CK(cudaMemsetAsync(c->ca.pen_count, 0, sizeof(unsigned long long) * 2 * c->pen_stride, c->stream));
@@ -2658,7 +2679,7 @@ int run_begin(crush_ctx* c) {
     c->last_tune_step = 0;
     c->run_open = true;
     c->sched_trial_pending = !c->tuning_fixed && c->n_hc >= SCHED_TRIAL_MIN_ELEMENTS;
-    if (!c->tuned && !c->tuning_fixed) {
+    if (!c->tuned && !c->tuning_fixed && !resident(c)) {
         st = autotune(c);
         if (st != CRUSH_OK) return st;
     }
@@ -2876,15 +2897,76 @@ int schedule_trial(crush_ctx* c) {
     return st;
 }
 
+// Contexts up to this size step in the resident kernel; larger ones by the
+// step graphs, whose streaming kernels use more of the memory bandwidth (us per
+// step, resident and graph: one crash of 90,578 elements 57.0 and 60.9, of
+// 140,602 77.5 and 80.5, of 200,949 101.0 and 100.1, of 278,960 118.8 and
+// 115.1; batches of 71,869 44.2 and 54.3, of 132,540 83.1 and 102.8, of 230,770
+// 147.6 and 152.4).
+constexpr long long RESIDENT_MAX_ELEMENTS = 160000;
+constexpr long long RESIDENT_MAX_STEPS = 1000;  // steps of one launch
+
+// Whether the context's steps run in the resident kernel: small, on the
+// automatic schedule, with nothing between the steps but what that kernel does.
+bool resident(const crush_ctx* c) {
+    return c->res_blocks > 0 && !c->tuning_fixed && !c->profiling && !c->ca.exhaustive && !c->frames_on &&
+           c->n_hc + c->n_sc_free <= RESIDENT_MAX_ELEMENTS && c->n_slots <= RESIDENT_MAX_SLOTS;
+}
+
+int resident_steps(crush_ctx* c, long long n) {
+    ResidentArgs a;
+    a.el = c->el_run();
+    for (int k = 0; k < 2; ++k) {
+        a.nd[k] = c->nd_step(k);
+        a.ca[k] = c->ca_step(k);
+    }
+    a.va = c->va;
+    a.ab = c->ab;
+    a.hist = c->hist;
+    a.ctls = c->ctls;
+    a.node_cn = c->node_cn;
+    a.done_out = c->slot_done;
+    a.mass_flag = c->mass_flag;
+    a.sync = c->res_sync;
+    a.step0 = c->host_step;
+    a.n_steps = (int)n;
+    a.adaptive = c->adaptive ? 1 : 0;
+    a.check_steps = c->check_steps;
+    a.any_separation = c->any_separation ? 1 : 0;
+    a.hist_on = c->hist_on ? 1 : 0;
+    a.n_slaves = c->n_slaves;
+    // One crash: every chunk, until it is done; more: those of running crashes.
+    a.lists = c->n_slots > 1 ? c->ab.lists : nullptr;
+    const long long ns[ACTIVE_SPACES] = {c->n_hc, c->n_all, c->n_nodes, c->ca.n_grid_slaves, c->ca.n_cnodes, c->ca.n_dyn_faces,
+                                         c->n_slaves, c->ca.n_st_slaves, c->n_sc_free};
+    for (int k = 0; k < ACTIVE_SPACES; ++k) {
+        a.space_off[k] = c->space_off_h[k];
+        a.space_n[k] = ns[k];
+    }
+    CK(cudaMemsetAsync(c->res_sync, 0, sizeof(ResidentSync), c->stream));
+    CK(launch_resident(c->stream, a, c->res_blocks));
+    c->res_used = true;
+    c->host_step += n;
+    c->last_was_graph = false;
+    return check_launch(c);
+}
+
 // Issue n_steps steps (graphs where the step index is on a period boundary).
 int issue_steps(crush_ctx* c, long long n_steps) {
     if (!c->run_open) return crush::fail(CRUSH_ERR_INVALID, "no open run (call crush_run_begin)");
     long long issued = 0;
     int st;
     while (issued < n_steps) {
+        if (resident(c) && !c->prologue_done && !c->contact_done) {
+            const long long n = std::min(n_steps - issued, RESIDENT_MAX_STEPS);
+            st = resident_steps(c, n);
+            if (st != CRUSH_OK) return st;
+            issued += n;
+            continue;
+        }
         // Crushed faces change the contact search as a run goes on: re-tune
         // every RETUNE_STEPS steps, on a graph boundary.
-        if (!c->tuning_fixed && c->host_step - c->last_tune_step >= RETUNE_STEPS && (c->period == 0 || c->host_step % c->period == 0)) {
+        if (!c->tuning_fixed && (!c->tuned || c->host_step - c->last_tune_step >= RETUNE_STEPS) && (c->period == 0 || c->host_step % c->period == 0)) {
             st = autotune(c);
             if (st != CRUSH_OK) return st;
             c->last_tune_step = c->host_step;
@@ -2929,7 +3011,10 @@ int issue_steps(crush_ctx* c, long long n_steps) {
 int all_done(crush_ctx* c, int* done) {
     c->done_h.resize(c->n_slots);
     CK(cudaMemcpyAsync(c->done_h.data(), c->slot_done, sizeof(int) * c->n_slots, cudaMemcpyDeviceToHost, c->stream));
+    ResidentSync rs{};
+    if (c->res_used) CK(cudaMemcpyAsync(&rs, c->res_sync, sizeof(rs), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (rs.error) return crush::fail(CRUSH_ERR_TIMEOUT, "a block of the resident step kernel gave up waiting at its barrier");
     int d = 1;
     for (int x : c->done_h) d &= x ? 1 : 0;
     *done = d;

@@ -13,7 +13,8 @@ constexpr int HIST_TREE = 256;  // columns of the part sums' tree
 // Whether slot `slot` takes a record now: its run's first record, a step
 // that is a multiple of history_steps, or the last step of a finished crash;
 // never twice at one step.
-__device__ __forceinline__ bool hist_due(const HistoryArrays& h, const Control* ctl, int slot, int mode) {
+template <class C>
+__device__ __forceinline__ bool hist_due(const HistoryArrays& h, const C* ctl, int slot, int mode) {
     if (!h.slot_on[slot]) return false;
     if (mode == HIST_INITIAL) return true;
     if (ctl->step == h.last_step[slot]) return false;

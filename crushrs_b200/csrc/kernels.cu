@@ -12,9 +12,10 @@
 //    CSR built at set-up, in f64 — the order and precision of the reference's
 //    serial scatter (src/kernel_simd.rs:573-586), so results are reproducible
 //    run to run and identical to the reference's summation.
-//  * Nothing here waits on another block or another GPU; every kernel is a
-//    plain data-parallel pass whose only cross-block interaction is an
-//    atomic integer count or an atomicMin on a bit pattern.
+//  * Every kernel but the resident step kernel (resident.cuh, a cooperative
+//    launch whose blocks meet at bounded barriers) is a plain data-parallel
+//    pass whose only cross-block interaction is an atomic integer count or an
+//    atomicMin on a bit pattern; nothing waits on another GPU.
 #include <cmath>
 #include <cfloat>
 #include <climits>
@@ -25,6 +26,7 @@
 #include "element.cuh"
 #include "kernels.cuh"
 #include "hencky.cuh"
+#include "history.cuh"
 
 namespace crush {
 
@@ -515,14 +517,16 @@ __global__ void k_incidence_split(long long nn, const uint32_t* __restrict__ rel
 #ifndef FORCES_MINB
 #define FORCES_MINB 2
 #endif
-__device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeArrays& nd, Control* ctls, int respect_done, long long e) {
+template <class C>
+__device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeArrays& nd, Control* ctls, const C* view, int respect_done,
+                                            long long e) {
     if (e >= el.n_hc) return;
     const long long S = el.stride;
     const float4 meta = ld_plane(el.planes, S, P_META, e);
     const float4 c0 = ld_plane(el.planes, S, P_CONN, e), c1 = ld_plane(el.planes, S, P_CONN + 1, e);
     const float4 st6 = el.state[6 * S + e];
     Control* ctl = ctls + __float_as_uint(meta.w);
-    if (respect_done && ctl->done) return;
+    if (respect_done && view[__float_as_uint(meta.w)].done) return;
     float4* out = reinterpret_cast<float4*>(el.corner + 24 * e);
     if (__float_as_uint(st6.y) != 0u) {  // already eroded: no force
         for (int k = 0; k < 6; ++k) out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -647,20 +651,21 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
 // mesh) the loads are all issued before the sum.
 // The node's slots come from its padded row of 8 (one round of loads
 // before the corner loads); a node with more than 8 uses the CSR.
-__device__ __forceinline__ double gather_component(const NodeArrays& nd, const float* __restrict__ corner, long long n, int d) {
+// (Plain loads of the corner forces: the resident step kernel writes them too.)
+__device__ __forceinline__ double gather_component(const NodeArrays& nd, const float* corner, long long n, int d) {
     const uint4 r0 = __ldg(nd.hc_ell + 2 * n), r1 = __ldg(nd.hc_ell + 2 * n + 1);
     double f = 0.0;
     if (r0.x != HC_ELL_MORE) {
         const uint32_t sl[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
         float c[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) c[j] = sl[j] != HC_ELL_NONE ? __ldg(corner + 3ull * sl[j] + d) : 0.f;  // slot = 8 e + corner
+        for (int j = 0; j < 8; ++j) c[j] = sl[j] != HC_ELL_NONE ? corner[3ull * sl[j] + d] : 0.f;  // slot = 8 e + corner
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             if (sl[j] != HC_ELL_NONE) f += (double)c[j];
     } else {
         const uint32_t b = __ldg(nd.hc_off + n), m = __ldg(nd.hc_off + n + 1) - b;
-        for (uint32_t k = 0; k < m; ++k) f += (double)__ldg(corner + 3ull * __ldg(nd.hc_slot + b + k) + d);
+        for (uint32_t k = 0; k < m; ++k) f += (double)corner[3ull * __ldg(nd.hc_slot + b + k) + d];
     }
     return f;
 }
@@ -681,7 +686,7 @@ __global__ void __launch_bounds__(FORCES_TPB, FORCES_MINB) k_forces(ElementArray
     if (!queue) {
         FOR_ACTIVE(el.act_hc, el.n_hc, 1, g) {
             int lane;
-            forces_body(el, nd, ctls, respect_done, active_entity(el.act_hc, g, 1, &lane));
+            forces_body(el, nd, ctls, ctls, respect_done, active_entity(el.act_hc, g, 1, &lane));
         }
         return;
     }
@@ -695,7 +700,7 @@ __global__ void __launch_bounds__(FORCES_TPB, FORCES_MINB) k_forces(ElementArray
         if (item >= chunks) break;
         for (int t = threadIdx.x; t < CHUNK; t += FORCES_TPB) {
             int lane;
-            forces_body(el, nd, ctls, respect_done, active_entity(el.act_hc, item * CHUNK + t, 1, &lane));
+            forces_body(el, nd, ctls, ctls, respect_done, active_entity(el.act_hc, item * CHUNK + t, 1, &lane));
         }
     }
     if (threadIdx.x == 0) {
@@ -711,13 +716,18 @@ __global__ void __launch_bounds__(FORCES_TPB, FORCES_MINB) k_forces(ElementArray
 // with the Hencky stress, one element per thread: F = Σ x_i ⊗ ∇N_i at
 // x = X + u; det F <= 0 erodes the element; f_i = (τ F⁻ᵀ V) ∇N_i plus the
 // hourglass force R Γᵀ with R = H (U Γ). Corner forces in f64.
+// WIDE: the loops unrolled, so that their loads are in flight together: for a
+// lone warp (the resident kernel); the streaming kernel keeps them rolled for
+// its occupancy.
 constexpr int SC_TPB = 128;
-__device__ __forceinline__ void scalar_force_body(const ElementArrays& el, const NodeArrays& nd, Control* ctls, int respect_done,
-                                                  long long i) {
+template <bool WIDE, class C>
+__device__ __forceinline__ void scalar_force_body(const ElementArrays& el, const NodeArrays& nd, Control* ctls, const C* view,
+                                                  int respect_done, long long i) {
     if (i >= el.sc_count) return;
     const long long e = el.sc_model[i];
-    Control* ctl = ctls + el.elem_slot[e];
-    if (respect_done && ctl->done) return;
+    const uint32_t slot = el.elem_slot[e];
+    Control* ctl = ctls + slot;
+    if (respect_done && view[slot].done) return;
     double* out = el.sc_corner + 24 * i;
     if (el.eroded_all[e]) {
         for (int k = 0; k < 24; ++k) out[k] = 0.0;
@@ -730,8 +740,13 @@ __device__ __forceinline__ void scalar_force_body(const ElementArrays& el, const
     // no per-node arrays stay live (the kernel's occupancy is register-bound).
     double f[9], q[12];
     for (int k = 0; k < 9; ++k) f[k] = 0.0;
+    uint32_t nid[8];
+    if (WIDE)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) nid[k] = el.conn_all[8 * e + k];
+#pragma unroll(WIDE ? 8 : 1)
     for (int k = 0; k < 8; ++k) {
-        const long long n = el.conn_all[8 * e + k];
+        const long long n = WIDE ? nid[k] : el.conn_all[8 * e + k];
         double xk[3], uk[3], gk[3], ak[4];
         for (int d = 0; d < 3; ++d) {
             uk[d] = nd.u[3 * n + d];
@@ -789,7 +804,7 @@ __global__ void __launch_bounds__(SC_TPB) k_forces_scalar(ElementArrays el, Node
         int lane;
         const long long t = active_entity(el.act_sc, g, 1, &lane);
         // a run lists the elastic elements with a free node; drop-in calls take them all
-        scalar_force_body(el, nd, ctls, respect_done, el.sc_list ? (t < el.n_sc ? (long long)el.sc_list[t] : el.sc_count) : t);
+        scalar_force_body<false>(el, nd, ctls, ctls, respect_done, el.sc_list ? (t < el.n_sc ? (long long)el.sc_list[t] : el.sc_count) : t);
     }
 }
 
@@ -994,7 +1009,8 @@ constexpr int DT_TPB = 256;
 // Per-element stability limit and mass-scaling surplus. The minimum per crash
 // slot is an atomicMin on the bit pattern of a non-negative double (order
 // independent); lanes of a warp that share a slot reduce first.
-__device__ __forceinline__ void elem_dt_body(const ElementArrays& el, const NodeArrays& nd, Control* ctls, const double* __restrict__ u,
+template <class C>
+__device__ __forceinline__ void elem_dt_body(const ElementArrays& el, const NodeArrays& nd, Control* ctls, const C* view, const double* u,
                                              int respect_done, long long e) {
     const int lane = threadIdx.x & 31;
     uint32_t slot = 0xffffffffu;
@@ -1005,7 +1021,7 @@ __device__ __forceinline__ void elem_dt_body(const ElementArrays& el, const Node
         const bool eroded = el.eroded_all[e] != 0;
         const uint4 q0 = __ldg(reinterpret_cast<const uint4*>(el.conn_all + 8 * e));
         const uint4 q1 = __ldg(reinterpret_cast<const uint4*>(el.conn_all + 8 * e) + 1);
-        Control* ctl = ctls + slot;
+        const C* ctl = view + slot;
         if (respect_done && ctl->done) {
             slot = 0xffffffffu;
         } else {
@@ -1052,15 +1068,12 @@ __global__ void __launch_bounds__(DT_TPB) k_elem_dt(ElementArrays el, NodeArrays
                                                     int respect_done, long long e_begin) {
     FOR_ACTIVE(el.act_all, el.n_all - e_begin, 1, g) {
         int lane;
-        elem_dt_body(el, nd, ctls, u, respect_done, e_begin + active_entity(el.act_all, g, 1, &lane));
+        elem_dt_body(el, nd, ctls, ctls, u, respect_done, e_begin + active_entity(el.act_all, g, 1, &lane));
     }
 }
 
-// The adaptive step decision of src/solver.rs:288-299, one thread per slot.
-__global__ void k_dt_finalize(Control* ctls, int n_slots, int* __restrict__ mass_flag) {
-    const int sl = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sl >= n_slots) return;
-    Control* ctl = ctls + sl;
+// The adaptive step decision of src/solver.rs:288-299 for one slot.
+__device__ __forceinline__ void dt_finalize_slot(Control* ctl, int* mass_flag) {
     if (ctl->done) return;
     const double dt_stable = __longlong_as_double((long long)ctl->dt_stable_bits);
     const double total = ctl->added_total_acc;
@@ -1077,12 +1090,17 @@ __global__ void k_dt_finalize(Control* ctls, int n_slots, int* __restrict__ mass
     }
     ctl->dt_cfl = ctl->dt_scale * fmin(dt_use, ctl->contact_dt);
 }
+__global__ void k_dt_finalize(Control* ctls, int n_slots, int* __restrict__ mass_flag) {
+    const int sl = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sl < n_slots) dt_finalize_slot(ctls + sl, mass_flag);
+}
 
 // Added nodal mass (element order, src/kernel.rs:246-255) and 1/(m + added).
-__device__ __forceinline__ void mass_scaling_body(const ElementArrays& el, const NodeArrays& nd, const Control* ctls, int force_apply,
+template <class C>
+__device__ __forceinline__ void mass_scaling_body(const ElementArrays& el, const NodeArrays& nd, const C* ctls, int force_apply,
                                                   long long n) {
     if (n >= nd.n || (!force_apply && !*nd.mass_flag)) return;
-    const Control* ctl = ctls + nd.node_slot[n];
+    const C* ctl = ctls + nd.node_slot[n];
     if (!force_apply && (ctl->done || !ctl->mass_scale_now)) return;
     const double floor = ctl->dt_floor;
     double add = 0.0;
@@ -1102,22 +1120,24 @@ __global__ void k_mass_scaling(ElementArrays el, NodeArrays nd, Control* ctls, i
     }
 }
 
+template <class C>
+__device__ __forceinline__ void nonfinite_body(const NodeArrays& nd, Control* ctls, const C* view, long long n) {
+    if (n >= nd.n) return;
+    Control* ctl = ctls + nd.node_slot[n];
+    if (view[nd.node_slot[n]].done) return;
+    if (!isfinite(nd.u[3 * n]) || !isfinite(nd.u[3 * n + 1]) || !isfinite(nd.u[3 * n + 2])) ctl->nonfinite = 1;
+}
 __global__ void k_nonfinite(NodeArrays nd, Control* ctls) {
     FOR_ACTIVE(nd.act_node, nd.n, 1, g) {
         int lane;
-        const long long n = active_entity(nd.act_node, g, 1, &lane);
-        if (n >= nd.n) continue;
-        Control* ctl = ctls + nd.node_slot[n];
-        if (ctl->done) continue;
-        if (!isfinite(nd.u[3 * n]) || !isfinite(nd.u[3 * n + 1]) || !isfinite(nd.u[3 * n + 2])) ctl->nonfinite = 1;
+        nonfinite_body(nd, ctls, ctls, active_entity(nd.act_node, g, 1, &lane));
     }
 }
 
 // The active chunk lists: thread per chunk (all entity spaces), a chunk is
 // active while any crash slot it holds is still running. One atomic per warp
 // and space.
-__global__ void k_build_active(ActiveBuild b, const Control* __restrict__ ctls) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void build_active_body(const ActiveBuild& b, const Control* ctls, long long t) {
     const int lane = threadIdx.x & 31;
     int space = -1;
     bool alive = false;
@@ -1136,6 +1156,9 @@ __global__ void k_build_active(ActiveBuild b, const Control* __restrict__ ctls) 
         base = __shfl_sync(grp, base, leader);
         b.lists[b.space_off[space] + base + __popc(grp & ((1u << lane) - 1u))] = (int)(t - b.space_off[space]);
     }
+}
+__global__ void k_build_active(ActiveBuild b, const Control* __restrict__ ctls) {
+    build_active_body(b, ctls, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // End of a step (src/solver.rs:344-345 plus the stop rules), one thread per slot.
@@ -1162,10 +1185,23 @@ __device__ void step_end_slot(Control* ctl, int sl, const ContactArrays& ca, con
     ctl->eroded_step = 0;
     ctl->mass_scale_now = 0;
     int hit = 0;
-    for (int c = ca.slot_contact_off[sl]; c < ca.slot_contact_off[sl + 1]; ++c) {
-        if (ca.counts_for_stop[c] && ca.pen_count[c] > 0) hit = 1;
-        ca.pen_count[c] = 0;
-        ca.pen_max_bits[c] = 0;
+    const int c0 = ca.slot_contact_off[sl], c1 = ca.slot_contact_off[sl + 1];
+    for (int c = c0; c < c1; c += 4) {  // four contacts' loads in flight (a head-on has four)
+        unsigned long long pen[4];
+        int counts[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            pen[k] = c + k < c1 ? ca.pen_count[c + k] : 0;
+            counts[k] = c + k < c1 ? ca.counts_for_stop[c + k] : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (counts[k] && pen[k] > 0) hit = 1;
+            if (c + k < c1) {
+                ca.pen_count[c + k] = 0;
+                ca.pen_max_bits[c + k] = 0;
+            }
+        }
     }
     if (hit) ctl->last_hit = ctl->step - 1;
     if (ctl->nonfinite) {
@@ -1287,7 +1323,8 @@ __device__ __forceinline__ int box_level(const ContactArrays& ca, int c, const d
 // the pass visits gets its cell record (level -1: no inserts), so the fill
 // pass, over the same faces, inserts exactly what was counted.
 constexpr int FACE_LANES = 4;
-__device__ __forceinline__ void contact_face_body(const ContactArrays& ca, const NodeArrays& nd, const Control* ctls, int c0,
+template <class C>
+__device__ __forceinline__ void contact_face_body(const ContactArrays& ca, const NodeArrays& nd, const C* ctls, int c0,
                                                   const uint32_t* __restrict__ face_list, long long n, int run_mode, int do_grid,
                                                   long long t, int lane) {
     if (t >= n) return;  // uniform over the face's lanes, as is every branch before the shuffles
@@ -1366,26 +1403,30 @@ __device__ __forceinline__ void contact_face_body(const ContactArrays& ca, const
 // list, same active chunks): the lanes split the face's stored cells and
 // place the face in each cell's bucket range from k_grid_alloc, which
 // returns every count to zero.
+__device__ __forceinline__ void contact_insert_body(const ContactArrays& ca, int c0, const uint32_t* face_list, long long n, long long t,
+                                                    int lane) {
+    if (t >= n) return;  // warp-uniform
+    const long long f = face_list ? (long long)face_list[t] : ca.face_off[c0] + t;
+    const int c = ca.face_contact[f];
+    const int tab = ca.tab_off[c];
+    if (ca.tab_off[c + 1] == tab) return;
+    const FaceCells fc = ca.cells[f];
+    if (fc.level < 0 || fc.level >= GRID_LEVELS) return;
+    const int local = (int)(f - ca.face_off[c]);
+    const unsigned mask = (unsigned)(ca.tab_off[c + 1] - tab - 1);
+    const int ni = fc.span[0], nj = fc.span[1], nk = fc.span[2];
+    for (int q = lane; q < ni * nj * nk; q += 32) {
+        const long long i = fc.lo[0] + q % ni, j = fc.lo[1] + (q / ni) % nj, k = fc.lo[2] + q / (ni * nj);
+        const int b = tab + (int)(cell_hash(i, j, k, fc.level) & mask);
+        const int pos = atomicSub(&ca.counts[b], 1) - 1;
+        ca.entries[ca.boff[b] + pos] = local;
+    }
+}
 __global__ void k_contact_insert(ContactArrays ca, int c0, const uint32_t* __restrict__ face_list, long long n, Active act) {
     FOR_ACTIVE(act, n, 32, g) {
         int lane;
-        const long long t = active_entity(act, g, 32, &lane);  // warp-uniform
-        if (t >= n) continue;
-        const long long f = face_list ? (long long)face_list[t] : ca.face_off[c0] + t;
-        const int c = ca.face_contact[f];
-        const int tab = ca.tab_off[c];
-        if (ca.tab_off[c + 1] == tab) continue;
-        const FaceCells fc = ca.cells[f];
-        if (fc.level < 0 || fc.level >= GRID_LEVELS) continue;
-        const int local = (int)(f - ca.face_off[c]);
-        const unsigned mask = (unsigned)(ca.tab_off[c + 1] - tab - 1);
-        const int ni = fc.span[0], nj = fc.span[1], nk = fc.span[2];
-        for (int q = lane; q < ni * nj * nk; q += 32) {
-            const long long i = fc.lo[0] + q % ni, j = fc.lo[1] + (q / ni) % nj, k = fc.lo[2] + q / (ni * nj);
-            const int b = tab + (int)(cell_hash(i, j, k, fc.level) & mask);
-            const int pos = atomicSub(&ca.counts[b], 1) - 1;
-            ca.entries[ca.boff[b] + pos] = local;
-        }
+        const long long t = active_entity(act, g, 32, &lane);
+        contact_insert_body(ca, c0, face_list, n, t, lane);
     }
 }
 
@@ -1402,8 +1443,8 @@ __global__ void __launch_bounds__(FACE_TPB) k_contact_faces(ContactArrays ca, No
 // Thread per dynamic bucket: its range in the contact's entries, allocated
 // with one atomic per warp (a warp's buckets belong to one table, since tables
 // are multiples of 1024 buckets).
-__global__ void k_grid_alloc(ContactArrays ca, int c0, int c1) {
-    const long long b = (long long)ca.tab_off[c0] + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void grid_alloc_body(const ContactArrays& ca, int c0, int c1, long long g) {
+    const long long b = (long long)ca.tab_off[c0] + g;
     const int lane = threadIdx.x & 31;
     if (b - lane >= ca.tab_off[c1]) return;  // warp-uniform
     // the warp's contact: the last c with tab_off[c] <= b (binary search)
@@ -1427,6 +1468,9 @@ __global__ void k_grid_alloc(ContactArrays ca, int c0, int c1) {
     base = __shfl_sync(0xffffffffu, base, 0);
     ca.boff[b] = (unsigned)(ca.ent_off[c] + base + incl - cnt);
     ca.blen[b] = cnt;
+}
+__global__ void k_grid_alloc(ContactArrays ca, int c0, int c1) {
+    grid_alloc_body(ca, c0, c1, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // src/contact.rs:29-43
@@ -1469,9 +1513,7 @@ __device__ __forceinline__ bool face_hit(const FaceGeo& g, const double* p, doub
 // big_best ends as the smallest big face that hits, whatever the order.
 constexpr int BIG_TPB = 128;
 constexpr int BIG_BLOCKS = 148 * 4;
-__global__ void __launch_bounds__(BIG_TPB) k_contact_big(ContactArrays ca, NodeArrays nd) {
-    __shared__ FaceGeo sg;
-    __shared__ double sbox[6];
+__device__ __forceinline__ void contact_big_block(const ContactArrays& ca, const NodeArrays& nd, FaceGeo& sg, double* sbox) {
     const int count = min(*ca.big_count, (int)ca.big_cap);
     for (int k = blockIdx.x; k < count; k += gridDim.x) {  // block-uniform
         const long long f = ca.big_faces[k];
@@ -1484,7 +1526,7 @@ __global__ void __launch_bounds__(BIG_TPB) k_contact_big(ContactArrays ca, NodeA
         const int local = (int)(f - ca.face_off[c]);
         const double md = ca.max_distance[c];
         const long long s1 = ca.slave_off[c + 1];
-        for (long long s = ca.slave_off[c] + threadIdx.x; s < s1; s += BIG_TPB) {
+        for (long long s = ca.slave_off[c] + threadIdx.x; s < s1; s += blockDim.x) {
             const long long n = ca.slaves[s];
             const double p[3] = {nd.pos[3 * n] + nd.u[3 * n], nd.pos[3 * n + 1] + nd.u[3 * n + 1], nd.pos[3 * n + 2] + nd.u[3 * n + 2]};
             if (!(p[0] >= sbox[0] && p[0] <= sbox[3] && p[1] >= sbox[1] && p[1] <= sbox[4] && p[2] >= sbox[2] && p[2] <= sbox[5])) continue;
@@ -1492,6 +1534,11 @@ __global__ void __launch_bounds__(BIG_TPB) k_contact_big(ContactArrays ca, NodeA
             if (face_hit(sg, p, md, &sd)) atomicMin(&ca.big_best[s], local);
         }
     }
+}
+__global__ void __launch_bounds__(BIG_TPB) k_contact_big(ContactArrays ca, NodeArrays nd) {
+    __shared__ FaceGeo sg;
+    __shared__ double sbox[6];
+    contact_big_block(ca, nd, sg, sbox);
 }
 
 // One reaction event of a hit: key 2s (the primary node's own +F) or 2s+1
@@ -1549,11 +1596,11 @@ __device__ __forceinline__ void record_hit(const ContactArrays& ca, long long s,
 // face the reference's in-order scan with `break` finds
 // (src/contact.rs:115-157). Lane 0 sets the node's big_best back to
 // BIG_NONE for the next search, also when its crash has stopped.
-template <int LANES>
-__device__ __forceinline__ void contact_slave_body(const ContactArrays& ca, const NodeArrays& nd, const Control* ctls, int c0, int c1,
+template <int LANES, class C>
+__device__ __forceinline__ int contact_slave_body(const ContactArrays& ca, const NodeArrays& nd, const C* ctls, int c0, int c1,
                                                    int run_mode, double dt_override, const double* __restrict__ masses, long long s,
-                                                   bool live, int lane) {
-    const Control* ctl = nullptr;
+                                                   bool live, int lane, double* sd_out = nullptr) {
+    const C* ctl = nullptr;
     bool reset_big = false;
     if (live) {
         const int c = ca.slave_contact[s];
@@ -1641,13 +1688,15 @@ __device__ __forceinline__ void contact_slave_body(const ContactArrays& ca, cons
         if (ob < best) { best = ob; best_sd = osd; }
     }
     if (reset_big) ca.big_best[s] = BIG_NONE;
-    if (!live || lane != 0) return;
+    if (!live || lane != 0) return -1;
     if (best == INT_MAX) {
         ca.hit[s] = -1;
-        return;
+        return -1;
     }
     ca.hit[s] = best;
     ca.hit_sd[s] = best_sd;
+    if (sd_out) *sd_out = best_sd;
+    return best;  // lane 0's: the face index, or -1
 }
 
 // run: the entries of `list` (grid_slaves or st_slaves, over their active
@@ -1733,6 +1782,17 @@ __global__ void __launch_bounds__(BRUTE_TPB) k_contact_brute(ContactArrays ca, N
 // thread per primary-node entry: run the search finished before (possibly
 // overlapping other work); this pass needs the step's dt and records the
 // reaction events and the penetration counters.
+template <class C>
+__device__ __forceinline__ void contact_force_body(const ContactArrays& ca, const C* ctls, int run_mode, double dt_override,
+                                                   const double* masses, int skip_fixed, int next_step, long long s, int lane) {
+    const int best = ca.hit[s];
+    if (best < 0) return;
+    const int c = ca.slave_contact[s];
+    const C* ctl = ctls + ca.contact_slot[c];
+    if (run_mode && ctl->done) return;
+    const double dt = dt_override > 0.0 ? dt_override : (next_step ? next_step_dt(ctl) : step_dt(ctl));
+    record_hit(ca, s, c, ca.slaves[s], best, ca.hit_sd[s], dt, masses, ca.geo[ca.face_off[c] + best], skip_fixed, lane);
+}
 __global__ void k_contact_force(ContactArrays ca, Control* ctls, int c0, int run_mode, double dt_override,
                                 const double* __restrict__ masses, long long n_slaves, int skip_fixed, int next_step) {
     const Active act = run_mode ? ca.act_allslave : Active{nullptr, nullptr};
@@ -1740,16 +1800,7 @@ __global__ void k_contact_force(ContactArrays ca, Control* ctls, int c0, int run
     FOR_ACTIVE(act, n_slaves, FORCE_LANES, g) {
         int lane;
         const long long e = active_entity(act, g, FORCE_LANES, &lane);
-        if (e >= n_slaves) continue;
-        const long long s = s0 + e;
-        const int best = ca.hit[s];
-        if (best < 0) continue;
-        const int c = ca.slave_contact[s];
-        const Control* ctl = ctls + ca.contact_slot[c];
-        if (run_mode && ctl->done) continue;
-        const double dt = dt_override > 0.0 ? dt_override : (next_step ? next_step_dt(ctl) : step_dt(ctl));
-        record_hit(ca, s, c, ca.slaves[s], best, ca.hit_sd[s], dt, masses,
-                   ca.geo[ca.face_off[c] + best], skip_fixed, lane);
+        if (e < n_slaves) contact_force_body(ca, ctls, run_mode, dt_override, masses, skip_fixed, next_step, s0 + e, lane);
     }
 }
 
@@ -1760,15 +1811,16 @@ __global__ void k_contact_force(ContactArrays ca, Control* ctls, int c0, int run
 // other gather, beside it on a second stream or after it on the same
 // stream, reads them to skip those nodes.
 constexpr int RESET_TPB = 512;
-__global__ void __launch_bounds__(RESET_TPB) k_contact_reset(ContactArrays ca) {
+__device__ __forceinline__ void contact_reset_block(const ContactArrays& ca) {
     const int count = *ca.gather_count;
-    for (int w = threadIdx.x; w < count; w += RESET_TPB) ca.ev_count[ca.gather_work[w]] = 0;
+    for (int w = threadIdx.x; w < count; w += blockDim.x) ca.ev_count[ca.gather_work[w]] = 0;
     __syncthreads();  // every thread has read the count
     if (threadIdx.x == 0) {
         *ca.ev_pool_n = 0;
         *ca.gather_count = 0;
     }
 }
+__global__ void __launch_bounds__(RESET_TPB) k_contact_reset(ContactArrays ca) { contact_reset_block(ca); }
 
 constexpr int GATHER_TPB = 128;
 constexpr int HEAVY_TPB = 256;
@@ -1792,38 +1844,14 @@ __device__ __forceinline__ void apply_event(bool face, double fx, double fy, dou
     }
 }
 
-// Ordered reaction gather, one thread per contact node. The node's events
-// carry keys 2s (own) and 2s+1 (face) of the global primary-node index s;
-// contacts are numbered in order and so are their entries, so ascending keys
-// are the order in which src/contact.rs:146-153 adds the reactions to f_ext,
-// contact after contact. Up to EV_CAP keys are sorted in registers (a
-// bitonic network) and their forces loaded together; a node with more goes
-// to k_contact_gather_heavy (the force pass listed it), which writes its
-// output; its count stays until k_contact_reset at the next pass, so this
-// gather skips it whichever kernel runs first. The gather zeroes the other
-// nodes' event counts for the next pass. In a run it also writes the node's
-// half-step u to u_next (fixed nodes and stopped crashes keep theirs), so
-// the next step's search can start before the half step.
-__device__ __forceinline__ void gather_body(const ContactArrays& ca, const NodeArrays& nd, const Control* ctls, int c0, int c1,
-                                            int run_mode, double* __restrict__ f_out, int skip_fixed, long long i) {
-    if (i >= ca.n_cnodes) return;
-    const long long n = ca.cnode[i];
-    if ((skip_fixed && nd.fixed[n]) || (run_mode && ctls[nd.node_slot[n]].done)) return;
-    if (!run_mode) {  // a drop-in call writes the nodes with a role in contacts [c0, c1)
-        bool touched = false;
-        for (uint32_t r = ca.cnode_off[i]; r < ca.cnode_off[i + 1]; ++r) {
-            const int c = ca.crole_contact[r];
-            touched |= c >= c0 && c < c1;
-        }
-        if (!touched) return;
-    }
-    const int cnt = ca.ev_count[i];
-    if (cnt > EV_CAP) return;  // k_contact_gather_heavy's node
-    double sx = 0.0, sy = 0.0, sz = 0.0;
+// The sum of contact node i's cnt <= EV_CAP events, in order; leaves its count at zero.
+// `row`: its key list (EV_CAP keys, read whatever the count).
+__device__ __forceinline__ void gather_events(const ContactArrays& ca, long long i, int cnt, const uint4* row, double& sx, double& sy,
+                                              double& sz) {
+    sx = sy = sz = 0.0;
     if (cnt > 0) {
         ca.ev_count[i] = 0;
         uint32_t k[EV_CAP];
-        const uint4* row = reinterpret_cast<const uint4*>(ca.ev_list + i * EV_CAP);
 #pragma unroll
         for (int q = 0; q < EV_CAP / 4; ++q) {
             const uint4 v = row[q];
@@ -1857,9 +1885,9 @@ __device__ __forceinline__ void gather_body(const ContactArrays& ca, const NodeA
                 for (int j = 0; j < 8; ++j) {
                     const long long e = (long long)(k[g + j] >> 1);
                     const bool ok = g + j < cnt;
-                    fx[j] = ok ? __ldg(ca.hit_force + 3 * e) : 0.0;
-                    fy[j] = ok ? __ldg(ca.hit_force + 3 * e + 1) : 0.0;
-                    fz[j] = ok ? __ldg(ca.hit_force + 3 * e + 2) : 0.0;
+                    fx[j] = ok ? ca.hit_force[3 * e] : 0.0;
+                    fy[j] = ok ? ca.hit_force[3 * e + 1] : 0.0;
+                    fz[j] = ok ? ca.hit_force[3 * e + 2] : 0.0;
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
@@ -1867,6 +1895,37 @@ __device__ __forceinline__ void gather_body(const ContactArrays& ca, const NodeA
             }
         }
     }
+}
+
+// Ordered reaction gather, one thread per contact node. The node's events
+// carry keys 2s (own) and 2s+1 (face) of the global primary-node index s;
+// contacts are numbered in order and so are their entries, so ascending keys
+// are the order in which src/contact.rs:146-153 adds the reactions to f_ext,
+// contact after contact. Up to EV_CAP keys are sorted in registers (a
+// bitonic network) and their forces loaded together; a node with more goes
+// to k_contact_gather_heavy (the force pass listed it), which writes its
+// output; its count stays until k_contact_reset at the next pass, so this
+// gather skips it whichever kernel runs first. The gather zeroes the other
+// nodes' event counts for the next pass. In a run it also writes the node's
+// half-step u to u_next (fixed nodes and stopped crashes keep theirs), so
+// the next step's search can start before the half step.
+__device__ __forceinline__ void gather_body(const ContactArrays& ca, const NodeArrays& nd, const Control* ctls, int c0, int c1,
+                                            int run_mode, double* __restrict__ f_out, int skip_fixed, long long i) {
+    if (i >= ca.n_cnodes) return;
+    const long long n = ca.cnode[i];
+    if ((skip_fixed && nd.fixed[n]) || (run_mode && ctls[nd.node_slot[n]].done)) return;
+    if (!run_mode) {  // a drop-in call writes the nodes with a role in contacts [c0, c1)
+        bool touched = false;
+        for (uint32_t r = ca.cnode_off[i]; r < ca.cnode_off[i + 1]; ++r) {
+            const int c = ca.crole_contact[r];
+            touched |= c >= c0 && c < c1;
+        }
+        if (!touched) return;
+    }
+    const int cnt = ca.ev_count[i];
+    if (cnt > EV_CAP) return;  // k_contact_gather_heavy's node
+    double sx, sy, sz;
+    gather_events(ca, i, cnt, reinterpret_cast<const uint4*>(ca.ev_list + i * EV_CAP), sx, sy, sz);
     f_out[3 * n] = sx;
     f_out[3 * n + 1] = sy;
     f_out[3 * n + 2] = sz;
@@ -1881,6 +1940,10 @@ __global__ void __launch_bounds__(GATHER_TPB) k_contact_gather(ContactArrays ca,
     }
 }
 
+// Barrier of the HEAVY_TPB threads that sum a heavy node (the first ones of a
+// larger block).
+__device__ __forceinline__ void heavy_sync() { asm volatile("bar.sync 1, %0;" ::"n"(HEAVY_TPB) : "memory"); }
+
 // Threads 0, 1 and 2 add, in order, component 0, 1 and 2 of the events
 // listed in keys[0, count) (ascending) to their running sum acc, the
 // forces fetched HEAVY_TPB at a time by the whole block. The components'
@@ -1894,7 +1957,7 @@ __device__ void heavy_sum(const ContactArrays& ca, const uint32_t* keys, int cou
             sf[threadIdx.x][1] = ca.hit_force[3 * e + 1];
             sf[threadIdx.x][2] = ca.hit_force[3 * e + 2];
         }
-        __syncthreads();
+        heavy_sync();
         if (threadIdx.x < 3) {
             const int m = min(HEAVY_TPB, count - b0);
             const int d = threadIdx.x;
@@ -1907,7 +1970,7 @@ __device__ void heavy_sum(const ContactArrays& ca, const uint32_t* keys, int cou
             }
             acc = a;
         }
-        __syncthreads();
+        heavy_sync();
     }
 }
 
@@ -1954,7 +2017,7 @@ __device__ void walk_node(const ContactArrays& ca, int c0, int c1, long long i, 
                 if (lane >= off) incl += y;
             }
             if (lane == 31) s_warp[warp] = incl;
-            __syncthreads();
+            heavy_sync();
             int before = 0, total = 0;
             for (int k = 0; k < HEAVY_TPB / 32; ++k) {
                 const int v = s_warp[k];
@@ -1968,7 +2031,7 @@ __device__ void walk_node(const ContactArrays& ca, int c0, int c1, long long i, 
                 if (own_j[j]) keys[pos++] = key;
                 for (int a = 0; a < m_j[j]; ++a) keys[pos++] = key + 1u;
             }
-            __syncthreads();
+            heavy_sync();
             heavy_sum(ca, keys, total, sf, acc);  // ends with a barrier: keys and s_warp are free again
         }
     }
@@ -1980,63 +2043,73 @@ __device__ void walk_node(const ContactArrays& ca, int c0, int c1, long long i, 
 // bitonic sort in shared memory and added in order. A node whose events do
 // not fit HEAVY_KEYS, or lost some to a full pool, is rebuilt by walk_node.
 // The nodes' event counts are left for k_contact_reset.
+struct HeavyShared {
+    uint32_t keys[HEAVY_BUF];
+    double sf[HEAVY_TPB][3];
+    int warp[HEAVY_TPB / 32];
+    int n;
+};
+// Node i with cnt events by one block: thread d < 3 returns component d of the sum.
+__device__ double heavy_node(const ContactArrays& ca, int c0, int c1, long long i, int cnt, HeavyShared& sh) {
+    uint32_t* keys = sh.keys;
+    double(*sf)[3] = sh.sf;
+    int* s_warp = sh.warp;
+    int& s_n = sh.n;
+    const long long n = ca.cnode[i];
+    double acc = 0.0;
+    bool walk = cnt > HEAVY_KEYS;
+    if (!walk) {
+        if (threadIdx.x == 0) s_n = 0;
+        heavy_sync();
+        for (int t = threadIdx.x; t < EV_CAP; t += HEAVY_TPB) keys[t] = ca.ev_list[i * EV_CAP + t];
+        const int np = (int)min((long long)*ca.ev_pool_n, ca.ev_pool_cap);
+        for (int p = threadIdx.x; p < np; p += HEAVY_TPB) {
+            const uint2 e = ca.ev_pool[p];
+            if (e.x == (uint32_t)i) {
+                const int q = EV_CAP + atomicAdd(&s_n, 1);
+                if (q < HEAVY_KEYS) keys[q] = e.y;
+            }
+        }
+        heavy_sync();
+        walk = EV_CAP + s_n != cnt;  // block-uniform
+    }
+    if (walk) {
+        heavy_sync();
+        walk_node(ca, c0, c1, i, n, keys, sf, s_warp, acc);
+    } else {
+        int P = EV_CAP;
+        while (P < cnt) P <<= 1;
+        for (int t = cnt + threadIdx.x; t < P; t += HEAVY_TPB) keys[t] = 0xFFFFFFFFu;
+        heavy_sync();
+        for (int size = 2; size <= P; size <<= 1)
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                for (int a = threadIdx.x; a < P; a += HEAVY_TPB) {
+                    const int b = a ^ stride;
+                    if (b > a) {
+                        const uint32_t x = keys[a], y = keys[b];
+                        const bool up = (a & size) == 0;
+                        if ((x > y) == up) {
+                            keys[a] = y;
+                            keys[b] = x;
+                        }
+                    }
+                }
+                heavy_sync();
+            }
+        heavy_sum(ca, keys, cnt, sf, acc);
+    }
+    return acc;
+}
+
 __global__ void __launch_bounds__(HEAVY_TPB) k_contact_gather_heavy(ContactArrays ca, NodeArrays nd, const Control* ctls, int c0, int c1,
                                                                     int run_mode, double* __restrict__ f_out) {
-    __shared__ uint32_t keys[HEAVY_BUF];
-    __shared__ double sf[HEAVY_TPB][3];
-    __shared__ int s_warp[HEAVY_TPB / 32];
-    __shared__ int s_n;
+    __shared__ HeavyShared sh;
     const int count = *ca.gather_count;
     for (int w = blockIdx.x; w < count; w += gridDim.x) {  // block-uniform
         const long long i = ca.gather_work[w];
-        const int cnt = ca.ev_count[i];  // final: the force pass is done
-        const long long n = ca.cnode[i];
-        double acc = 0.0;  // thread d < 3: component d of the running sum
-        bool walk = cnt > HEAVY_KEYS;
-        if (!walk) {
-            if (threadIdx.x == 0) s_n = 0;
-            __syncthreads();
-            for (int t = threadIdx.x; t < EV_CAP; t += HEAVY_TPB) keys[t] = ca.ev_list[i * EV_CAP + t];
-            const int np = (int)min((long long)*ca.ev_pool_n, ca.ev_pool_cap);
-            for (int p = threadIdx.x; p < np; p += HEAVY_TPB) {
-                const uint2 e = ca.ev_pool[p];
-                if (e.x == (uint32_t)i) {
-                    const int q = EV_CAP + atomicAdd(&s_n, 1);
-                    if (q < HEAVY_KEYS) keys[q] = e.y;
-                }
-            }
-            __syncthreads();
-            walk = EV_CAP + s_n != cnt;  // block-uniform
-        }
-        if (walk) {
-            __syncthreads();
-            walk_node(ca, c0, c1, i, n, keys, sf, s_warp, acc);
-        } else {
-            int P = EV_CAP;
-            while (P < cnt) P <<= 1;
-            for (int t = cnt + threadIdx.x; t < P; t += HEAVY_TPB) keys[t] = 0xFFFFFFFFu;
-            __syncthreads();
-            for (int size = 2; size <= P; size <<= 1)
-                for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                    for (int a = threadIdx.x; a < P; a += HEAVY_TPB) {
-                        const int b = a ^ stride;
-                        if (b > a) {
-                            const uint32_t x = keys[a], y = keys[b];
-                            const bool up = (a & size) == 0;
-                            if ((x > y) == up) {
-                                keys[a] = y;
-                                keys[b] = x;
-                            }
-                        }
-                    }
-                    __syncthreads();
-                }
-            heavy_sum(ca, keys, cnt, sf, acc);
-        }
-        if (threadIdx.x < 3) {
-            f_out[3 * n + threadIdx.x] = acc;
-        }
-        __syncthreads();  // every thread is done with s_n and the shared buffers
+        const double acc = heavy_node(ca, c0, c1, i, ca.ev_count[i], sh);  // the count is final: the force pass is done
+        if (threadIdx.x < 3) f_out[3 * (long long)ca.cnode[i] + threadIdx.x] = acc;
+        __syncthreads();  // every thread is done with the shared buffers
     }
 }
 
@@ -2044,7 +2117,7 @@ __global__ void __launch_bounds__(HEAVY_TPB) k_contact_gather_heavy(ContactArray
 // FP64 vehicle reductions (delta-v, crush, separation rule), one block per
 // vehicle (or per vehicle slice), fixed summation order.
 // ---------------------------------------------------------------------------
-constexpr int VEH_TPB = 256;
+constexpr int VEH_TPB = HEAVY_TPB;
 
 __global__ void __launch_bounds__(VEH_TPB) k_vehicle_sums(VehicleArrays va, const double* __restrict__ mass, const double* __restrict__ v,
                                                           const double* __restrict__ v0, double* __restrict__ out) {
@@ -2089,10 +2162,9 @@ __device__ __forceinline__ long long vx_blocks_of(long long len) {
 // blocks per vehicle, each over a contiguous slice of the vehicle's nodes
 // (the launch has va.vx_blocks, the largest count; surplus blocks write zero
 // partials); k_step_end adds the partials in block order.
-__global__ void __launch_bounds__(VEH_TPB) k_vehicle_vx(VehicleArrays va, const double* __restrict__ mass, const double* __restrict__ v,
-                                                        Control* ctls) {
-    __shared__ double sm[VEH_TPB], sp[VEH_TPB];
-    const int veh = blockIdx.x / va.vx_blocks, b = blockIdx.x % va.vx_blocks;
+__device__ __forceinline__ void vehicle_vx_block(const VehicleArrays& va, const double* mass, const double* v, Control* ctls, int unit,
+                                                 double* sm, double* sp) {
+    const int veh = unit / va.vx_blocks, b = unit % va.vx_blocks;
     Control* ctl = ctls + va.slot[veh];
     const int lv = va.local[veh];
     if (ctl->done || lv >= 4) return;
@@ -2108,18 +2180,30 @@ __global__ void __launch_bounds__(VEH_TPB) k_vehicle_vx(VehicleArrays va, const 
     }
     sm[threadIdx.x] = m_acc;
     sp[threadIdx.x] = p_acc;
-    __syncthreads();
+    heavy_sync();
     for (int w = VEH_TPB / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) {
             sm[threadIdx.x] += sm[threadIdx.x + w];
             sp[threadIdx.x] += sp[threadIdx.x + w];
         }
-        __syncthreads();
+        heavy_sync();
     }
     if (threadIdx.x == 0) {
         ctl->vx_part[lv][b][0] = sm[0];
         ctl->vx_part[lv][b][1] = sp[0];
     }
+}
+__global__ void __launch_bounds__(VEH_TPB) k_vehicle_vx(VehicleArrays va, const double* __restrict__ mass, const double* __restrict__ v,
+                                                        Control* ctls) {
+    __shared__ double sm[VEH_TPB], sp[VEH_TPB];
+    vehicle_vx_block(va, mass, v, ctls, blockIdx.x, sm, sp);
+}
+
+#include "resident.cuh"
+
+__global__ void k_node_cn(const uint32_t* __restrict__ cnode, long long i0, long long i1, uint32_t* __restrict__ node_cn) {
+    const long long i = i0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < i1) node_cn[cnode[i]] = (uint32_t)i;
 }
 
 }  // namespace
@@ -2127,6 +2211,22 @@ __global__ void __launch_bounds__(VEH_TPB) k_vehicle_vx(VehicleArrays va, const 
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
+int resident_blocks(int device, int n_sms) {
+    int coop = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_steps<RES_SMALL>, RES_SMALL, 0) != cudaSuccess || per_sm < 1) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_steps<RES_LARGE>, RES_LARGE, 0) != cudaSuccess || per_sm < 1) return 0;
+    return n_sms;
+}
+cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks) {
+    void* args[] = {const_cast<ResidentArgs*>(&a)};
+    if (a.el.n_hc > 32 * (RES_SMALL / 32) * (long long)blocks)
+        return cudaLaunchCooperativeKernel(k_steps<RES_LARGE>, dim3((unsigned)blocks), dim3(RES_LARGE), args, 0, s);
+    return cudaLaunchCooperativeKernel(k_steps<RES_SMALL>, dim3((unsigned)blocks), dim3(RES_SMALL), args, 0, s);
+}
+void launch_node_cn(cudaStream_t s, const uint32_t* cnode, long long i0, long long i1, uint32_t* node_cn) {
+    if (i1 > i0) k_node_cn<<<(unsigned)blocks_for(i1 - i0, TPB), TPB, 0, s>>>(cnode, i0, i1, node_cn);
+}
 void launch_setup_geometry(cudaStream_t s, long long e_begin, long long n_all, const double* pos, const uint32_t* conn_all,
                            const int32_t* part, const double* mat, const int64_t* hc_index, const uint32_t* elem_slot, long long stride,
                            float4* planes, double* volume, double* lumped, double* dt_factor, double* elem_mass, int* bad,

@@ -83,6 +83,14 @@ struct FaceCells {
     int level;
 };
 
+// An entry of an exhaustively searched contact with what its search looks up.
+struct alignas(32) BruteEntry {
+    uint32_t s, node;   // primary-node entry and its node
+    int contact, slot;
+    int face0, n_faces; // the contact's faces
+    int pad[2];
+};
+
 // Contact runtime arrays (all contacts concatenated).
 struct FaceGeo {
     double x[4][3];
@@ -96,6 +104,7 @@ struct FaceGeo {
 // rest in a shared pool; CN_FIXED marks a fixed node in slave_cn / face_cn.
 constexpr int EV_CAP = 16;
 constexpr uint32_t CN_FIXED = 0x80000000u;
+constexpr uint32_t CN_NONE = 0xFFFFFFFFu;  // node_cn of a node without a contact role
 // Dynamic grids are hashed and hierarchical: level l has cells of size
 // cell * 4^l, and a face goes into the finest level where its key box covers
 // at most LEVEL_CELL_BUDGET cells. Buckets are exact CSR ranges rebuilt every
@@ -185,6 +194,8 @@ struct ContactArrays {
     // the others are listed for the lane-parallel search.
     const int* brute_contacts;
     int n_brute;
+    const BruteEntry* brute_entries;
+    long long n_brute_entries;
     int brute_max_faces;        // most faces of a listed contact (its shared-memory stage)
     const double* st_box;       // 6 per contact: union of a static contact's key boxes (lo xyz, hi xyz)
     const uint32_t* grid_slaves;  // entries searched with the tuned lane count (dynamic grids, no usable grid)
@@ -413,6 +424,40 @@ struct FrameArrays {
 };
 // One frame of every slot that is due (modes as for the histories).
 void launch_frames(cudaStream_t s, const FrameArrays& f, const double* u, const Control* ctls, int mode);
+
+// ---- Resident step kernel (resident.cuh) ----
+struct ResidentSync {
+    unsigned count, gen;  // grid barrier: arrivals, barriers with a serial part passed
+    int error;            // a block gave up waiting at a barrier
+    int pad;
+};
+constexpr int RESIDENT_MAX_SLOTS = 128;  // crashes of one launch (their control views are in shared memory)
+struct ResidentArgs {
+    ElementArrays el;     // el_run
+    NodeArrays nd[2];     // of even and odd steps (nd_step)
+    ContactArrays ca[2];  // of even and odd steps (ca_step)
+    VehicleArrays va;
+    ActiveBuild ab;
+    HistoryArrays hist;
+    Control* ctls;
+    const uint32_t* node_cn;  // per node: its contact node, or CN_NONE
+    int* done_out;
+    int* mass_flag;
+    ResidentSync* sync;
+    long long step0;
+    int n_steps;
+    int adaptive, check_steps, any_separation, hist_on;
+    long long n_slaves;
+    const int* lists;     // active chunk lists (ab.lists), or null: every chunk of every space
+    long long space_off[ACTIVE_SPACES];
+    long long space_n[ACTIVE_SPACES];
+};
+// Steps [step0, step0 + n_steps) of every slot in one cooperative launch of
+// `blocks` blocks (at most resident_blocks: those that fit the device at once).
+int resident_blocks(int device, int n_sms);
+cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks);
+// node_cn of contact nodes [i0, i1).
+void launch_node_cn(cudaStream_t s, const uint32_t* cnode, long long i0, long long i1, uint32_t* node_cn);
 
 // The call's kernels on `s`; every count is within the limits above.
 void launch_contact_static(cudaStream_t s, StaticContactScratch* sc, long long n_model_nodes, const double* pos, const double* u,
