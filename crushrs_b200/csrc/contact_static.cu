@@ -8,7 +8,7 @@
 // device together with the context's unique id; a call from another context
 // on that device (a driver-API context, or the primary context recreated
 // after cudaDeviceReset) resolves it again. After that a call is argument
-// checks and six kernel launches on the caller's stream: no device or host
+// checks and four kernel launches on the caller's stream: no device or host
 // allocation, no copy, no synchronisation.
 #include <cuda.h>  // CUcontext and CUresult only: the driver calls go through cudaGetDriverEntryPoint
 

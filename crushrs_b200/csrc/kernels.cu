@@ -2556,195 +2556,206 @@ void launch_contact_geometry(cudaStream_t s, const ContactArrays& ca, const Node
 namespace crush {
 namespace {
 
-constexpr int STATIC_TPB = 256;
-constexpr int STATIC_ONE_BLOCK = 1024;
-constexpr int STATIC_TILE = 256;
+// Four launches: faces and filter box, search and forces, sums, stores. A call
+// is bound by their latency (a chain of reads in each, one warp's instruction
+// stream): 304 faces and 120 nodes take 33.8 us; a box, a compaction of
+// the hits in blocks of their own and faces tested 32 at a time to the end took
+// 56.3 us in six launches.
+constexpr int STATIC_TPB = 128;
+constexpr int STATIC_SEARCH_TPB = 64;
+constexpr int STATIC_TILE = STATIC_TPB;
+static_assert(STATIC_TILE % 8 == 0, "hits are compared eight at a time");
 
-// Single block: validates node ids, resets the record's counters and forms
-// the filter box: the faces' bounding box at the reference positions grown by
-// max_distance.
-__global__ void __launch_bounds__(STATIC_ONE_BLOCK) k_static_prepare(StaticContactScratch* sc, long long n_model,
-                                                                      const double* __restrict__ pos, long long n_nodes,
-                                                                      const uint32_t* __restrict__ nodes, long long n_faces,
-                                                                      const uint32_t* __restrict__ faces, double md) {
-    __shared__ double s_lo[3][STATIC_ONE_BLOCK / 32], s_hi[3][STATIC_ONE_BLOCK / 32];
-    __shared__ int s_bad;
-    if (threadIdx.x == 0) s_bad = 0;
-    __syncthreads();
-    double lo[3] = {CUDART_INF, CUDART_INF, CUDART_INF}, hi[3] = {-CUDART_INF, -CUDART_INF, -CUDART_INF};
+// Whether a block of the face pass met an id out of range, and the filter box
+// (the faces' bounding box at the reference positions grown by max_distance):
+// every block of a later pass combines the face pass's parts itself.
+__device__ __forceinline__ bool static_bad(const StaticContactScratch* sc, int parts) {
     int bad = 0;
-    for (long long k = threadIdx.x; k < 4 * n_faces; k += blockDim.x) {
-        const uint32_t n = faces[k];
-        if (n >= n_model) {
-            bad = 1;
-            continue;
-        }
-        for (int d = 0; d < 3; ++d) {
-            const double p = pos[3 * (long long)n + d];
-            lo[d] = fmin(lo[d], p);
-            hi[d] = fmax(hi[d], p);
-        }
-    }
-    for (long long k = threadIdx.x; k < n_nodes; k += blockDim.x)
-        if (nodes[k] >= n_model) bad = 1;
-    if (bad) atomicOr(&s_bad, 1);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int d = 0; d < 3; ++d)
-        for (int off = 16; off > 0; off >>= 1) {
-            lo[d] = fmin(lo[d], __shfl_down_sync(0xffffffffu, lo[d], off));
-            hi[d] = fmax(hi[d], __shfl_down_sync(0xffffffffu, hi[d], off));
-        }
-    if (lane == 0)
-        for (int d = 0; d < 3; ++d) {
-            s_lo[d][w] = lo[d];
-            s_hi[d][w] = hi[d];
-        }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int d = 0; d < 3; ++d) {
-            double a = s_lo[d][0], b = s_hi[d][0];
-            for (int k = 1; k < (int)(blockDim.x / 32); ++k) {
-                a = fmin(a, s_lo[d][k]);
-                b = fmax(b, s_hi[d][k]);
-            }
-            sc->box_lo[d] = a + -md;
-            sc->box_hi[d] = b + md;
-        }
-        sc->pen_count = 0;
-        sc->pen_max_bits = 0;
-        sc->n_hits = 0;
-        sc->error = s_bad;
-    }
+    for (int k = threadIdx.x; k < parts; k += blockDim.x) bad |= sc->part_bad[k];
+    return __syncthreads_or(bad) != 0;
 }
 
-// Face geometry at X + u, thread per face (the arithmetic of k_contact_faces).
-__global__ void k_static_faces(StaticContactScratch* sc, const double* __restrict__ pos, const double* __restrict__ u,
-                               long long n_faces, const uint32_t* __restrict__ faces, double md) {
+// Thread per face: its node ids checked, its geometry at X + u (the arithmetic
+// of k_contact_faces) and the block's part of the box; the primary-node ids
+// are checked by the grid's threads in turn, and the counters start at zero.
+__global__ void __launch_bounds__(STATIC_FACE_TPB) k_static_faces(StaticContactScratch* sc, long long n_model,
+                                                                   const double* __restrict__ pos, const double* __restrict__ u,
+                                                                   long long n_nodes, const uint32_t* __restrict__ nodes, long long n_faces,
+                                                                   const uint32_t* __restrict__ faces, double md) {
+    __shared__ double s_box[6][STATIC_FACE_TPB / 32];
     const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= n_faces || sc->error) return;
-    FaceGeo g;
-    for (int k = 0; k < 4; ++k) {
-        const long long n = faces[4 * f + k];
-        for (int d = 0; d < 3; ++d) g.x[k][d] = pos[3 * n + d] + u[3 * n + d];
-    }
-    double e1[3], e2[3];
-    for (int d = 0; d < 3; ++d) {
-        e1[d] = g.x[1][d] - g.x[0][d];
-        e2[d] = g.x[2][d] - g.x[0][d];
-    }
-    const double nx = e1[1] * e2[2] - e1[2] * e2[1];
-    const double ny = e1[2] * e2[0] - e1[0] * e2[2];
-    const double nz = e1[0] * e2[1] - e1[1] * e2[0];
-    const double len = sqrt(nx * nx + ny * ny + nz * nz);
-    g.n[0] = nx / len;
-    g.n[1] = ny / len;
-    g.n[2] = nz / len;
-    for (int d = 0; d < 3; ++d) {
-        g.c[d] = (((g.x[0][d] + g.x[1][d]) + g.x[2][d]) + g.x[3][d]) / 4.0;
-        double lo = g.x[0][d], hi = g.x[0][d];
-        for (int k = 1; k < 4; ++k) {
-            lo = fmin(lo, g.x[k][d]);
-            hi = fmax(hi, g.x[k][d]);
+    int bad = 0;
+    for (long long k = f; k < n_nodes; k += (long long)gridDim.x * blockDim.x) bad |= nodes[k] >= n_model;
+    double box[6] = {CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF};  // lo, -hi: minima all
+    if (f < n_faces) {
+        uint32_t n[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            n[k] = faces[4 * f + k];
+            bad |= n[k] >= n_model;
         }
-        g.lo[d] = lo + -md;
-        g.hi[d] = hi + md;
+        if (!bad) {
+            FaceGeo g;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const double p = pos[3 * (long long)n[k] + d];
+                    box[d] = fmin(box[d], p);
+                    box[3 + d] = fmin(box[3 + d], -p);
+                    g.x[k][d] = p + u[3 * (long long)n[k] + d];
+                }
+            double e1[3], e2[3];
+            for (int d = 0; d < 3; ++d) {
+                e1[d] = g.x[1][d] - g.x[0][d];
+                e2[d] = g.x[2][d] - g.x[0][d];
+            }
+            const double nx = e1[1] * e2[2] - e1[2] * e2[1];
+            const double ny = e1[2] * e2[0] - e1[0] * e2[2];
+            const double nz = e1[0] * e2[1] - e1[1] * e2[0];
+            const double len = sqrt(nx * nx + ny * ny + nz * nz);
+            g.n[0] = nx / len;
+            g.n[1] = ny / len;
+            g.n[2] = nz / len;
+            for (int d = 0; d < 3; ++d) {
+                g.c[d] = (((g.x[0][d] + g.x[1][d]) + g.x[2][d]) + g.x[3][d]) / 4.0;
+                double lo = g.x[0][d], hi = g.x[0][d];
+                for (int k = 1; k < 4; ++k) {
+                    lo = fmin(lo, g.x[k][d]);
+                    hi = fmax(hi, g.x[k][d]);
+                }
+                g.lo[d] = lo + -md;
+                g.hi[d] = hi + md;
+            }
+            sc->geo[f] = g;
+        }
     }
-    sc->geo[f] = g;
+#pragma unroll
+    for (int d = 0; d < 6; ++d)
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) box[d] = fmin(box[d], __shfl_down_sync(0xffffffffu, box[d], off));
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int d = 0; d < 6; ++d) s_box[d][threadIdx.x >> 5] = box[d];
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x < 6) {
+        double m = s_box[threadIdx.x][0];
+        for (int k = 1; k < STATIC_FACE_TPB / 32; ++k) m = fmin(m, s_box[threadIdx.x][k]);
+        sc->part_box[threadIdx.x][blockIdx.x] = m;
+    }
+    if (threadIdx.x == 0) {
+        sc->part_bad[blockIdx.x] = bad;
+        if (blockIdx.x == 0) {
+            sc->pen_count = 0;
+            sc->pen_max_bits = 0;
+        }
+    }
 }
 
 // Warp per primary-node entry: the filter, then the smallest face index that
 // passes the narrow test (the face the reference's in-order scan finds) and
-// the penalty force on it.
-__global__ void k_static_search(StaticContactScratch* sc, const double* __restrict__ pos, const double* __restrict__ u,
-                                const double* __restrict__ masses, long long n_nodes, const uint32_t* __restrict__ nodes,
-                                const double* __restrict__ node_scale, long long n_faces, double stiffness, double md,
-                                double dt) {
-    const long long s = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // warp-uniform
+// the penalty force on it. The faces' boxes are tested 32 x STATIC_BATCH at a
+// time; the faces of a batch that pass are listed, their narrow tests run one
+// per lane, and the first batch with a hit ends the search.
+constexpr int STATIC_BATCH = 4;
+__global__ void __launch_bounds__(STATIC_SEARCH_TPB) k_static_search(StaticContactScratch* sc, int parts, const double* __restrict__ pos,
+                                                                     const double* __restrict__ u, const double* __restrict__ masses,
+                                                                     long long n_nodes, const uint32_t* __restrict__ nodes,
+                                                                     const double* __restrict__ node_scale, long long n_faces,
+                                                                     double stiffness, double md, double dt) {
+    __shared__ uint8_t s_cand[STATIC_SEARCH_TPB / 32][32 * STATIC_BATCH];
     const int lane = threadIdx.x & 31;
-    if (s >= n_nodes || sc->error) return;
-    const long long n = nodes[s];
+    uint8_t* cand = s_cand[threadIdx.x >> 5];
+    const long long s = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // warp-uniform
+    const long long n = s < n_nodes ? nodes[s] : 0;
+    // every warp combines the parts itself: no block-wide wait
+    double box[6] = {CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF, CUDART_INF};
+    int bad = 0;
+    for (int k = lane; k < parts; k += 32) {
+        bad |= sc->part_bad[k];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) box[d] = fmin(box[d], sc->part_box[d][k]);
+    }
+    if (s >= n_nodes || __any_sync(0xffffffffu, bad)) return;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int d = 0; d < 6; ++d) box[d] = fmin(box[d], __shfl_xor_sync(0xffffffffu, box[d], off));
     bool keep = true;
+    double p[3];
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
         const double x = pos[3 * n + d];
-        if (!(x >= sc->box_lo[d] && x <= sc->box_hi[d])) keep = false;
+        if (!(x >= box[d] + -md && x <= -box[3 + d] + md)) keep = false;
+        p[d] = x + u[3 * n + d];
     }
-    if (!keep) {
-        if (lane == 0) sc->hit[s] = -1;
-        return;
-    }
-    const double p[3] = {pos[3 * n] + u[3 * n], pos[3 * n + 1] + u[3 * n + 1], pos[3 * n + 2] + u[3 * n + 2]};
-    int best = INT_MAX;
-    double best_sd = 0.0, sd;
-    for (long long f = lane; f < n_faces; f += 32)
-        if (f < best && face_hit(sc->geo[f], p, md, &sd)) {
-            best = (int)f;
-            best_sd = sd;
+    int first = INT_MAX;
+    double sd = 0.0;
+    for (long long f0 = 0; keep && f0 < n_faces && first == INT_MAX; f0 += 32 * STATIC_BATCH) {  // warp-uniform
+        bool in[STATIC_BATCH];
+#pragma unroll
+        for (int k = 0; k < STATIC_BATCH; ++k) {
+            const long long f = f0 + 32 * k + lane;
+            const FaceGeo& g = sc->geo[f < n_faces ? f : 0];
+            const double l0 = g.lo[0], l1 = g.lo[1], l2 = g.lo[2], h0 = g.hi[0], h1 = g.hi[1], h2 = g.hi[2];
+            in[k] = f < n_faces && !(p[0] < l0 || p[0] > h0 || p[1] < l1 || p[1] > h1 || p[2] < l2 || p[2] > h2);
         }
-    for (int off = 16; off > 0; off >>= 1) {
-        const int ob = __shfl_down_sync(0xffffffffu, best, off);
-        const double osd = __shfl_down_sync(0xffffffffu, best_sd, off);
-        if (ob < best) {
-            best = ob;
-            best_sd = osd;
+        int count = 0;
+#pragma unroll
+        for (int k = 0; k < STATIC_BATCH; ++k) {
+            const unsigned m = __ballot_sync(0xffffffffu, in[k]);
+            if (in[k]) cand[count + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(32 * k + lane);
+            count += __popc(m);
         }
+        __syncwarp();
+        int best = INT_MAX;
+        double best_sd = 0.0;
+        for (int k = lane; k < count; k += 32) {  // ascending: a lane's first hit is its smallest
+            const int f = (int)f0 + cand[k];
+            if (face_hit(sc->geo[f], p, md, &best_sd)) {
+                best = f;
+                break;
+            }
+        }
+        __syncwarp();  // the list is free again
+        first = __reduce_min_sync(0xffffffffu, best);
+        if (first != INT_MAX) sd = __shfl_sync(0xffffffffu, best_sd, __ffs(__ballot_sync(0xffffffffu, best == first)) - 1);
     }
     if (lane != 0) return;
-    if (best == INT_MAX) {
+    if (first == INT_MAX) {
         sc->hit[s] = -1;
         return;
     }
     const double scale = node_scale ? node_scale[s] : 1.0;
     const double m = masses[n];
-    const double depth = fmin(-best_sd, 0.1 * md);
+    const double depth = fmin(-sd, 0.1 * md);
     const double k_pen = fmin(stiffness * scale, 0.1 * m / (dt * dt));
     const double mag = fmin(k_pen * depth, m * 1.0e5);
-    const FaceGeo& g = sc->geo[best];
-    sc->hit[s] = best;
+    const FaceGeo& g = sc->geo[first];
+    sc->hit[s] = first;
     sc->hit_force[3 * s] = mag * g.n[0];
     sc->hit_force[3 * s + 1] = mag * g.n[1];
     sc->hit_force[3 * s + 2] = mag * g.n[2];
     atomicAdd(&sc->pen_count, 1ull);
-    atomicMax(&sc->pen_max_bits, (unsigned long long)__double_as_longlong(-best_sd + 0.0));  // + 0.0: no -0.0 bits
-}
-
-// Single block: the entries that hit, compacted in entry order.
-__global__ void __launch_bounds__(STATIC_ONE_BLOCK) k_static_compact(StaticContactScratch* sc, long long n_nodes) {
-    __shared__ int s_warp[STATIC_ONE_BLOCK / 32];
-    __shared__ int s_base;
-    if (sc->error) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (threadIdx.x == 0) s_base = 0;
-    __syncthreads();
-    for (long long c0 = 0; c0 < n_nodes; c0 += blockDim.x) {
-        const long long i = c0 + threadIdx.x;
-        const bool flag = i < n_nodes && sc->hit[i] >= 0;
-        const unsigned ballot = __ballot_sync(0xffffffffu, flag);
-        if (lane == 0) s_warp[w] = __popc(ballot);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int k = 0; k < nw; ++k) {
-            if (k < w) before += s_warp[k];
-            total += s_warp[k];
-        }
-        if (flag) sc->hit_list[s_base + before + __popc(ballot & ((1u << lane) - 1u))] = (int)i;
-        __syncthreads();
-        if (threadIdx.x == 0) s_base += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) sc->n_hits = s_base;
+    atomicMax(&sc->pen_max_bits, (unsigned long long)__double_as_longlong(-sd + 0.0));  // + 0.0: no -0.0 bits
 }
 
 // Thread per node occurrence (the primary-node entries, then the face
 // corners): the node's force value after this contact, adding the hits in
 // entry order — +F for its own hit, -F/4 per corner it fills on a hit face —
 // starting from the value in f_accum (src/contact.rs:146-153).
-__global__ void __launch_bounds__(STATIC_TPB) k_static_occ(StaticContactScratch* sc, long long n_nodes, const uint32_t* __restrict__ nodes,
-                                                           long long n_faces, const uint32_t* __restrict__ faces,
-                                                           const double* __restrict__ f_accum) {
+// The hits are listed in entry order by each block for itself, a tile of
+// entries at a time.
+__global__ void __launch_bounds__(STATIC_TPB) k_static_occ(StaticContactScratch* sc, int parts, long long n_nodes,
+                                                           const uint32_t* __restrict__ nodes, long long n_faces,
+                                                           const uint32_t* __restrict__ faces, const double* __restrict__ f_accum) {
     __shared__ uint32_t t_node[STATIC_TILE];
-    __shared__ uint32_t t_face[STATIC_TILE][4];
+    __shared__ uint4 t_face[STATIC_TILE];
     __shared__ double t_f[STATIC_TILE][3];
-    if (sc->error) return;  // grid-uniform
+    __shared__ int s_warp[STATIC_TPB / 32];
+    static_assert(STATIC_TILE == STATIC_TPB, "an entry per thread");
+    if (static_bad(sc, parts)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long n_occ = n_nodes + 4 * n_faces;
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = o < n_occ;
@@ -2755,32 +2766,53 @@ __global__ void __launch_bounds__(STATIC_TPB) k_static_occ(StaticContactScratch*
         v1 = f_accum[3 * n + 1];
         v2 = f_accum[3 * n + 2];
     }
-    const int H = sc->n_hits;
-    for (int t0 = 0; t0 < H; t0 += STATIC_TILE) {
-        const int nt = min(STATIC_TILE, H - t0);
+    for (long long s0 = 0; s0 < n_nodes; s0 += STATIC_TILE) {
+        const long long s = s0 + threadIdx.x;
+        const int fc = s < n_nodes ? sc->hit[s] : -1;
+        const unsigned ballot = __ballot_sync(0xffffffffu, fc >= 0);
+        if (lane == 0) s_warp[w] = __popc(ballot);
         __syncthreads();
-        for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-            const int s = sc->hit_list[t0 + k];
-            const long long fc = sc->hit[s];
-            t_node[k] = nodes[s];
-            for (int j = 0; j < 4; ++j) t_face[k][j] = faces[4 * fc + j];
-            for (int d = 0; d < 3; ++d) t_f[k][d] = sc->hit_force[3 * s + d];
+        int at = 0, nt = 0;
+#pragma unroll
+        for (int k = 0; k < STATIC_TPB / 32; ++k) {
+            const int c = s_warp[k];
+            at += k < w ? c : 0;
+            nt += c;
+        }
+        if (fc >= 0) {
+            at += __popc(ballot & ((1u << lane) - 1u));
+            t_node[at] = nodes[s];
+            t_face[at] = make_uint4(faces[4ll * fc], faces[4ll * fc + 1], faces[4ll * fc + 2], faces[4ll * fc + 3]);
+            for (int d = 0; d < 3; ++d) t_f[at][d] = sc->hit_force[3 * s + d];
         }
         __syncthreads();
-        if (live)
-            for (int k = 0; k < nt; ++k) {
+        // Few hits touch a node: eight are compared at a time, and those that
+        // do are added in order.
+        for (int k0 = 0; live && k0 < nt; k0 += 8) {
+            unsigned touch = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint4 q = t_face[k0 + j];
+                const uint32_t m = (uint32_t)n;
+                if (k0 + j < nt && (t_node[k0 + j] == m || q.x == m || q.y == m || q.z == m || q.w == m)) touch |= 1u << j;
+            }
+            for (; touch; touch &= touch - 1) {
+                const int k = k0 + __ffs(touch) - 1;
                 if (t_node[k] == (uint32_t)n) {
                     v0 += t_f[k][0];
                     v1 += t_f[k][1];
                     v2 += t_f[k][2];
                 }
-                for (int j = 0; j < 4; ++j)
-                    if (t_face[k][j] == (uint32_t)n) {
-                        v0 -= 0.25 * t_f[k][0];
-                        v1 -= 0.25 * t_f[k][1];
-                        v2 -= 0.25 * t_f[k][2];
-                    }
+                const uint4 q = t_face[k];
+                const int corners = (q.x == (uint32_t)n) + (q.y == (uint32_t)n) + (q.z == (uint32_t)n) + (q.w == (uint32_t)n);
+                for (int j = 0; j < corners; ++j) {
+                    v0 -= 0.25 * t_f[k][0];
+                    v1 -= 0.25 * t_f[k][1];
+                    v2 -= 0.25 * t_f[k][2];
+                }
             }
+        }
+        __syncthreads();  // the tile is free again
     }
     if (live) {
         sc->occ[3 * o] = v0;
@@ -2791,11 +2823,11 @@ __global__ void __launch_bounds__(STATIC_TPB) k_static_occ(StaticContactScratch*
 
 // Thread per occurrence: store the node's new value (every occurrence of a
 // node holds the same value, so repeated stores agree); thread 0 reports.
-__global__ void k_static_write(StaticContactScratch* sc, long long n_nodes, const uint32_t* __restrict__ nodes, long long n_faces,
-                               const uint32_t* __restrict__ faces, double* __restrict__ f_accum, int64_t* stats_count,
+__global__ void k_static_write(StaticContactScratch* sc, int parts, long long n_nodes, const uint32_t* __restrict__ nodes,
+                               long long n_faces, const uint32_t* __restrict__ faces, double* __restrict__ f_accum, int64_t* stats_count,
                                double* stats_max, int* stats_status) {
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int err = sc->error;
+    const bool err = static_bad(sc, parts);
     if (o == 0) {
         if (stats_count) *stats_count = err ? 0 : (int64_t)sc->pen_count;
         if (stats_max) *stats_max = err ? 0.0 : __longlong_as_double((long long)sc->pen_max_bits);
@@ -2814,16 +2846,16 @@ void launch_contact_static(cudaStream_t s, StaticContactScratch* sc, long long n
                            const double* masses, long long n_nodes, const uint32_t* nodes, const double* node_scale,
                            long long n_faces, const uint32_t* faces, double stiffness, double max_distance, double dt,
                            double* f_accum, int64_t* stats_count, double* stats_max, int* stats_status) {
-    k_static_prepare<<<1, STATIC_ONE_BLOCK, 0, s>>>(sc, n_model_nodes, pos, n_nodes, nodes, n_faces, faces, max_distance);
-    if (n_faces > 0) k_static_faces<<<(unsigned)blocks_for(n_faces, STATIC_TPB), STATIC_TPB, 0, s>>>(sc, pos, u, n_faces, faces, max_distance);
+    const int parts = (int)blocks_for(n_faces > 0 ? n_faces : 1, STATIC_FACE_TPB);
+    k_static_faces<<<(unsigned)parts, STATIC_FACE_TPB, 0, s>>>(sc, n_model_nodes, pos, u, n_nodes, nodes, n_faces, faces, max_distance);
     if (n_nodes > 0)
-        k_static_search<<<(unsigned)blocks_for(n_nodes * 32, STATIC_TPB), STATIC_TPB, 0, s>>>(
-            sc, pos, u, masses, n_nodes, nodes, node_scale, n_faces, stiffness, max_distance, dt);
-    k_static_compact<<<1, STATIC_ONE_BLOCK, 0, s>>>(sc, n_nodes);
+        k_static_search<<<(unsigned)blocks_for(n_nodes * 32, STATIC_SEARCH_TPB), STATIC_SEARCH_TPB, 0, s>>>(
+            sc, parts, pos, u, masses, n_nodes, nodes, node_scale, n_faces, stiffness, max_distance, dt);
     const long long n_occ = n_nodes + 4 * n_faces;
-    if (n_occ > 0) k_static_occ<<<(unsigned)blocks_for(n_occ, STATIC_TPB), STATIC_TPB, 0, s>>>(sc, n_nodes, nodes, n_faces, faces, f_accum);
+    if (n_occ > 0)
+        k_static_occ<<<(unsigned)blocks_for(n_occ, STATIC_TPB), STATIC_TPB, 0, s>>>(sc, parts, n_nodes, nodes, n_faces, faces, f_accum);
     k_static_write<<<(unsigned)blocks_for(n_occ > 0 ? n_occ : 1, STATIC_TPB), STATIC_TPB, 0, s>>>(
-        sc, n_nodes, nodes, n_faces, faces, f_accum, stats_count, stats_max, stats_status);
+        sc, parts, n_nodes, nodes, n_faces, faces, f_accum, stats_count, stats_max, stats_status);
 }
 
 }  // namespace crush

@@ -332,17 +332,17 @@ void launch_gather_ux(cudaStream_t s, long long n, const uint32_t* nodes, const 
 // the bounding-box filter) and STATIC_MAX_FACES faces per call.
 constexpr int STATIC_MAX_NODES = 16384;
 constexpr int STATIC_MAX_FACES = 16384;
+constexpr int STATIC_FACE_TPB = 128;
+constexpr int STATIC_MAX_PARTS = STATIC_MAX_FACES / STATIC_FACE_TPB;
 constexpr int STATIC_MAX_OCC = STATIC_MAX_NODES + 4 * STATIC_MAX_FACES;  // node occurrences
 struct StaticContactScratch {
     FaceGeo geo[STATIC_MAX_FACES];
     double hit_force[3 * STATIC_MAX_NODES];
     double occ[3 * STATIC_MAX_OCC];    // new force value of the node of each occurrence
     int hit[STATIC_MAX_NODES];         // face hit by each primary node entry, or -1
-    int hit_list[STATIC_MAX_NODES];    // entries that hit, in entry order
-    double box_lo[3], box_hi[3];       // primary-node filter box (reference positions)
+    double part_box[6][STATIC_MAX_PARTS];  // per block of the face pass: its faces' reference box (lo xyz, hi xyz)
+    int part_bad[STATIC_MAX_PARTS];    // per block: it met a node id out of range (nothing is written then)
     unsigned long long pen_count, pen_max_bits;
-    int n_hits;
-    int error;                         // 1: a node id was out of range (nothing is written)
 };
 
 // ---- Time histories (part states and accelerometer samples) ----

@@ -496,7 +496,7 @@ int crush_run_issue(crush_ctx* ctx, int64_t n_steps);
  * calls that can overlap in time (other streams or threads without ordering
  * between them) race and corrupt each other's results: serialise them.
  *
- * Asynchronous: six kernel launches on `stream` (a cudaStream_t; NULL = the
+ * Asynchronous: four kernel launches on `stream` (a cudaStream_t; NULL = the
  * legacy default stream) of the current device, no copy, no synchronisation.
  * The host checks only sizes and arguments; node ids are checked on the
  * device: an id >= n_model_nodes writes nothing and sets stats->status to
