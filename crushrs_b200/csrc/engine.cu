@@ -1474,14 +1474,12 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     std::vector<uint32_t> gslaves, stslaves;
     std::vector<BruteEntry> bents;
     std::vector<uint8_t> is_brute(std::max(K, 1), 0);
-    int brute_max = c->ca.brute_max_faces;
     for (int q = 0; q < K; ++q) {
         const bool st_grid = st_tab_off[q + 1] > st_tab_off[q];
         const bool grid = tab_off[q + 1] > tab_off[q] || st_grid;
         if (!grid && face_off[q + 1] - face_off[q] <= 255 && slave_off[q + 1] > slave_off[q]) {
             brute.push_back(K0 + q);
             is_brute[q] = 1;
-            brute_max = std::max(brute_max, face_off[q + 1] - face_off[q]);
             for (int e = slave_off[q]; e < slave_off[q + 1]; ++e)
                 bents.push_back(BruteEntry{(uint32_t)e, slaves[e - base[0].slave], K0 + q, contact_slot[q], face_off[q],
                                            face_off[q + 1] - face_off[q], {0, 0}});
@@ -1899,7 +1897,6 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     ca.n_dyn_faces = tot.dyn;
     ca.n_cnodes = tot.cnode;
     ca.n_brute += (int)brute.size();
-    ca.brute_max_faces = std::max(brute_max, 1);
     ca.n_grid_slaves = (long long)c->grid_slaves_h.size();
     ca.n_st_slaves = (long long)c->st_slaves_h.size();
     ca.is_brute_h = c->is_brute_h.data();

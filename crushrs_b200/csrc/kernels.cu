@@ -1311,19 +1311,21 @@ __device__ __forceinline__ int box_level(const ContactArrays& ca, int c, const d
     return GRID_LEVELS;
 }
 
-// Thread per face: the face's geometry at X + u. The faces are
-// face_list[0, n) when face_list is given (the run: moving faces only), else
-// face_off[c0] + [0, n).
-// FACE_LANES lanes per face: its geometry at X + u, and — when the search
-// builds the dynamic grids (do_grid) and the face's contact has one — its key
+// A face's geometry at X + u. The faces are face_list[0, n) when face_list is
+// given (the run: moving faces only), else face_off[c0] + [0, n).
+// LANES lanes per face: FACE_LANES when the search builds the dynamic grids
+// (do_grid), for the faces whose contact has one — the face's key
 // box (lane t takes triangle t, the quad combines them), grid level and
 // cells, stored for the fill pass, with one count per cell added to the
 // cell's bucket (the lanes split the cells); a face whose box fits no level
 // is listed as a big face with its key box. Every face of a grid contact that
 // the pass visits gets its cell record (level -1: no inserts), so the fill
 // pass, over the same faces, inserts exactly what was counted.
+// One lane per face when no contact has a grid: the geometry is one chain that
+// more lanes only repeat (39,680 faces on the SMs the element kernel leaves: 77 us,
+// 158 us with four).
 constexpr int FACE_LANES = 4;
-template <class C>
+template <int LANES, class C>
 __device__ __forceinline__ void contact_face_body(const ContactArrays& ca, const NodeArrays& nd, const C* ctls, int c0,
                                                   const uint32_t* __restrict__ face_list, long long n, int run_mode, int do_grid,
                                                   long long t, int lane) {
@@ -1341,14 +1343,14 @@ __device__ __forceinline__ void contact_face_body(const ContactArrays& ca, const
     FaceGeo g;
     face_geometry(ca, nd, f, md, g);
     {
-        constexpr int per = (int)(sizeof(FaceGeo) / sizeof(double)) / FACE_LANES;
+        constexpr int per = (int)(sizeof(FaceGeo) / sizeof(double)) / LANES;
         const double* src = reinterpret_cast<const double*>(&g);
         double* dst = reinterpret_cast<double*>(ca.geo + f);
 #pragma unroll
         for (int k = 0; k < (int)(sizeof(FaceGeo) / sizeof(double)); ++k)
             if (k / per == lane) dst[k] = src[k];
     }
-    if (!grid) return;
+    if (LANES == 1 || !grid) return;
     double rlo[3] = {1e300, 1e300, 1e300}, rhi[3] = {-1e300, -1e300, -1e300};
     int perp = key_box_triangle(g.x, g.n, g.c, lane, rlo, rhi) == KEY_TRI_PERP ? 1 : 0;
 #pragma unroll
@@ -1430,13 +1432,14 @@ __global__ void k_contact_insert(ContactArrays ca, int c0, const uint32_t* __res
     }
 }
 
+template <int LANES>
 __global__ void __launch_bounds__(FACE_TPB) k_contact_faces(ContactArrays ca, NodeArrays nd, Control* ctls, int c0,
                                                             const uint32_t* __restrict__ face_list, long long n, int run_mode, int do_grid,
                                                             Active act) {
-    FOR_ACTIVE(act, n, FACE_LANES, g) {
+    FOR_ACTIVE(act, n, LANES, g) {
         int lane;
-        const long long t = active_entity(act, g, FACE_LANES, &lane);
-        contact_face_body(ca, nd, ctls, c0, face_list, n, run_mode, do_grid, t, lane);
+        const long long t = active_entity(act, g, LANES, &lane);
+        contact_face_body<LANES>(ca, nd, ctls, c0, face_list, n, run_mode, do_grid, t, lane);
     }
 }
 
@@ -1718,24 +1721,26 @@ constexpr int ST_LANES = 2;  // lanes per entry of a static-grid contact (a box 
 
 // Contacts searched exhaustively (fewer faces than the grid threshold), a
 // few blocks per contact (gridDim.y, brute_split) sharing its primary-node
-// entries: each block stages the contact's face geometry in shared memory
-// and each thread scans the faces in order for one primary node and stops at
-// the first hit, as src/contact.rs:115-157 does.
+// entries: each lane marks those of its faces whose box holds its primary node,
+// then runs their narrow tests in order and stops at the first hit, as
+// src/contact.rs:115-157 does. Bound by the f64 narrow tests. The geometry is
+// read through L1, not staged in shared memory: an SM that holds a persistent
+// block of the element kernel keeps that kernel's shared-memory split, so a
+// block with 48 KB could not start beside it and the search waited for the
+// element kernel's end (512 crashes, 1.06 M elements: the search starts 80 us into
+// the element kernel instead of 60 us after it, 364 instead of 400 us per step
+// with the one-lane face pass).
 constexpr int BRUTE_TPB = 128;
-constexpr int BRUTE_MAX_FACES = 255;  // 255 x 192 B fits the default 48 KB of shared memory
+constexpr int BRUTE_MAX_FACES = 255;  // a lane's faces fit the 64 bits of its mask with 4 lanes
 template <int BRUTE_LANES>
 __global__ void __launch_bounds__(BRUTE_TPB) k_contact_brute(ContactArrays ca, NodeArrays nd, Control* ctls, const int* __restrict__ list,
                                                             int single, int run_mode, double dt_override, const double* __restrict__ masses) {
-    extern __shared__ double sbuf[];
-    FaceGeo* sgeo = reinterpret_cast<FaceGeo*>(sbuf);
     const int c = list ? list[blockIdx.x] : single;
     const Control* ctl = ctls + ca.contact_slot[c];
     if (run_mode && ctl->done) return;  // block-uniform
     const long long fb = ca.face_off[c];
     const int nf = (int)(ca.face_off[c + 1] - fb);
-    const double* src = reinterpret_cast<const double*>(ca.geo + fb);
-    for (int k = threadIdx.x; k < nf * (int)(sizeof(FaceGeo) / sizeof(double)); k += blockDim.x) sbuf[k] = src[k];
-    __syncthreads();
+    const FaceGeo* geo = ca.geo + fb;
     const double md = ca.max_distance[c];
     // BRUTE_LANES lanes per primary node, each scanning every BRUTE_LANES-th
     // face in order up to its first hit; the smallest hit index wins.
@@ -1752,12 +1757,21 @@ __global__ void __launch_bounds__(BRUTE_TPB) k_contact_brute(ContactArrays ca, N
         if (live) {
             n = ca.slaves[s];
             const double p[3] = {nd.pos[3 * n] + nd.u[3 * n], nd.pos[3 * n + 1] + nd.u[3 * n + 1], nd.pos[3 * n + 2] + nd.u[3 * n + 2]};
-            for (int f = lane; f < nf; f += BRUTE_LANES)
-                if (face_hit(sgeo[f], p, md, &sd)) {
+            unsigned long long mask = 0;
+#pragma unroll 4
+            for (int f = lane, k = 0; f < nf; f += BRUTE_LANES, ++k) {
+                const double* b = geo[f].lo;  // lo, then hi
+                const double l0 = b[0], l1 = b[1], l2 = b[2], h0 = b[3], h1 = b[4], h2 = b[5];
+                if (!(p[0] < l0 || p[0] > h0 || p[1] < l1 || p[1] > h1 || p[2] < l2 || p[2] > h2)) mask |= 1ull << k;
+            }
+            for (; mask; mask &= mask - 1) {
+                const int f = lane + BRUTE_LANES * (__ffsll((long long)mask) - 1);
+                if (face_hit(geo[f], p, md, &sd)) {
                     best = f;
                     best_sd = sd;
                     break;
                 }
+            }
         }
 #pragma unroll
         for (int off = BRUTE_LANES / 2; off > 0; off >>= 1) {
@@ -2385,7 +2399,7 @@ void launch_vehicle_vx(cudaStream_t s, const VehicleArrays& va, const double* ma
 }
 
 // Blocks per exhaustively searched contact: enough for about four blocks per
-// SM over all such contacts (each block stages the contact's faces), at most 8.
+// SM over all such contacts, at most 8.
 unsigned brute_split(long long n_brute) {
     const long long target = 4 * 148;
     return (unsigned)std::min<long long>(8, std::max<long long>(1, (target + n_brute - 1) / std::max<long long>(n_brute, 1)));
@@ -2396,16 +2410,16 @@ unsigned brute_split(long long n_brute) {
 // choice finds the same first hit.
 template <int LANES>
 void launch_brute(cudaStream_t s, const ContactArrays& ca, const NodeArrays& nd, Control* ctls, const int* list, int single, unsigned n,
-                  unsigned split, size_t smem) {
-    k_contact_brute<LANES><<<dim3(n, split), BRUTE_TPB, smem, s>>>(ca, nd, ctls, list, single, list ? 1 : 0, 0.0, nullptr);
+                  unsigned split) {
+    k_contact_brute<LANES><<<dim3(n, split), BRUTE_TPB, 0, s>>>(ca, nd, ctls, list, single, list ? 1 : 0, 0.0, nullptr);
 }
 void launch_brute_any(cudaStream_t s, const ContactArrays& ca, const NodeArrays& nd, Control* ctls, const int* list, int single,
-                      long long n_brute, size_t smem) {
+                      long long n_brute) {
     if (n_brute * 8 <= 4 * 148) {
         const unsigned split = (unsigned)std::min<long long>(16, std::max<long long>(1, (16 * 148 + n_brute - 1) / std::max<long long>(n_brute, 1)));
-        launch_brute<16>(s, ca, nd, ctls, list, single, (unsigned)std::max<long long>(n_brute, 1), split, smem);
+        launch_brute<16>(s, ca, nd, ctls, list, single, (unsigned)std::max<long long>(n_brute, 1), split);
     } else {
-        launch_brute<4>(s, ca, nd, ctls, list, single, (unsigned)n_brute, brute_split(n_brute), smem);
+        launch_brute<4>(s, ca, nd, ctls, list, single, (unsigned)n_brute, brute_split(n_brute));
     }
 }
 
@@ -2422,9 +2436,14 @@ void launch_contact_search(cudaStream_t s, const ContactArrays& ca, const NodeAr
     // Every search starts from clear grid bookkeeping (levels in use, entry
     // cursors, big-face list), whatever ran before it.
     cudaMemsetAsync(ca.grid_state, 0, sizeof(int) * (2 * (size_t)ca.contact_room + 1), s);
-    if (n_list > 0)
-        k_contact_faces<<<active_grid(n_list, FACE_LANES, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, ctls, c0, list, n_list,
-                                                                                               run_mode, do_grid, act);
+    if (n_list > 0) {
+        if (do_grid)
+            k_contact_faces<FACE_LANES><<<active_grid(n_list, FACE_LANES, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, ctls, c0, list,
+                                                                                                               n_list, run_mode, 1, act);
+        else
+            k_contact_faces<1><<<active_grid(n_list, 1, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, ctls, c0, list, n_list, run_mode, 0,
+                                                                                             act);
+    }
     if (do_grid) {
         k_grid_alloc<<<(unsigned)blocks_for(bk1 - bk0, TPB), TPB, 0, s>>>(ca, c0, c1);
         if (n_list > 0) {
@@ -2435,9 +2454,9 @@ void launch_contact_search(cudaStream_t s, const ContactArrays& ca, const NodeAr
     // Exhaustive contacts: a block each (run: the listed ones; drop-in: the one contact if it is one).
     if (!ca.exhaustive) {
         if (run_mode && ca.n_brute > 0)
-            launch_brute_any(s, ca, nd, ctls, ca.brute_contacts, 0, ca.n_brute, sizeof(FaceGeo) * ca.brute_max_faces);
+            launch_brute_any(s, ca, nd, ctls, ca.brute_contacts, 0, ca.n_brute);
         if (!run_mode && c1 == c0 + 1 && ca.is_brute_h && ca.is_brute_h[c0]) {
-            launch_brute_any(s, ca, nd, ctls, nullptr, c0, 1, sizeof(FaceGeo) * BRUTE_MAX_FACES);
+            launch_brute_any(s, ca, nd, ctls, nullptr, c0, 1);
             n_slaves = 0;
         }
         if (run_mode) n_slaves = ca.n_grid_slaves;
@@ -2538,8 +2557,8 @@ void launch_contact_geometry(cudaStream_t s, const ContactArrays& ca, const Node
     (void)f0;
     if (c1 <= c0 || n_faces <= 0) return;
     (void)c1;
-    k_contact_faces<<<active_grid(n_faces, FACE_LANES, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, nullptr, c0, nullptr, n_faces,
-                                                                                            0, 0, Active{nullptr, nullptr});
+    k_contact_faces<1><<<active_grid(n_faces, 1, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, nullptr, c0, nullptr, n_faces, 0, 0,
+                                                                                      Active{nullptr, nullptr});
 }
 
 }  // namespace crush

@@ -196,7 +196,6 @@ struct ContactArrays {
     int n_brute;
     const BruteEntry* brute_entries;
     long long n_brute_entries;
-    int brute_max_faces;        // most faces of a listed contact (its shared-memory stage)
     const double* st_box;       // 6 per contact: union of a static contact's key boxes (lo xyz, hi xyz)
     const uint32_t* grid_slaves;  // entries searched with the tuned lane count (dynamic grids, no usable grid)
     long long n_grid_slaves;

@@ -429,11 +429,18 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                 const long long k = entity(8, t, 1, &l);
                 scalar_force_body<true>(el, nd, ctls, view, 1, k < el.n_sc ? (long long)el.sc_list[k] : el.sc_count);
             });
-        deal(tasks(5, FACE_LANES), [&](int t) {
-            int l;
-            const long long k = entity(5, t, FACE_LANES, &l);
-            contact_face_body(ca, nd, view, 0, ca.dyn_faces, ca.n_dyn_faces, 1, ca.n_buckets > 0 ? 1 : 0, k, l);
-        });
+        if (ca.n_buckets > 0)
+            deal(tasks(5, FACE_LANES), [&](int t) {
+                int l;
+                const long long k = entity(5, t, FACE_LANES, &l);
+                contact_face_body<FACE_LANES>(ca, nd, view, 0, ca.dyn_faces, ca.n_dyn_faces, 1, 1, k, l);
+            });
+        else
+            deal(tasks(5, 1), [&](int t) {
+                int l;
+                const long long k = entity(5, t, 1, &l);
+                contact_face_body<1>(ca, nd, view, 0, ca.dyn_faces, ca.n_dyn_faces, 1, 0, k, l);
+            });
         if (!(go = barrier(&s_state))) break;
         deal.base = 0;
 
