@@ -16,6 +16,7 @@
 //    launch whose blocks meet at bounded barriers) is a plain data-parallel
 //    pass whose only cross-block interaction is an atomic integer count or an
 //    atomicMin on a bit pattern; nothing waits on another GPU.
+#include <atomic>
 #include <cmath>
 #include <cfloat>
 #include <climits>
@@ -799,6 +800,158 @@ __device__ __forceinline__ void scalar_force_body(const ElementArrays& el, const
     }
 }
 
+// The same element on eight lanes, a node each, for few elements (a lone
+// thread's element is bound by its instruction stream: some 4000 f64
+// operations and library calls in a chain, 16 us in the resident kernel). The
+// lanes share the sums over the nodes (a component of F or q per lane, in node
+// order), the inverse, the rows of H and the nodes' forces through `sh`
+// (OCT_SHARED doubles per element); hencky_elastic_oct splits the stress. Each
+// value is computed by the operations of scalar_force_body. All 32 lanes
+// call, with i = -1 for none. A step of the two-part pair (1008 elastic
+// elements) takes 21 us, 27 us with a thread per element.
+constexpr int OCT_SHARED = 104;
+template <class C>
+__device__ __forceinline__ void scalar_force_oct(const ElementArrays& el, const NodeArrays& nd, Control* ctls, const C* view,
+                                                 int respect_done, long long i, double* sh) {
+    const int l = threadIdx.x & 7;
+    bool live = i >= 0 && i < el.sc_count;
+    const long long S = el.sc_stride;
+    const double* G = el.sc_geo;
+    long long e = 0;
+    uint32_t slot = 0;
+    if (live) {
+        e = el.sc_model[i];
+        slot = el.elem_slot[e];
+        if (respect_done && view[slot].done) live = false;
+    }
+    double* out = el.sc_corner + 24 * i;
+    if (live && el.eroded_all[e]) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) out[3 * l + d] = 0.0;
+        live = false;
+    }
+    // this lane's node, and every load of the element that depends on nothing
+    double u[3] = {0.0, 0.0, 0.0}, x[3] = {0.0, 0.0, 0.0}, gk[3] = {0.0, 0.0, 0.0}, ak[4] = {0.0, 0.0, 0.0, 0.0};
+    double h0[12], h1[12], vol = 0.0, youngs = 1.0, poisson = 0.0;
+    const int row1 = 8 + (l & 3);  // lanes 0-3 take rows 8-11 as well
+#pragma unroll
+    for (int c = 0; c < 12; ++c) h0[c] = h1[c] = 0.0;
+    if (live) {
+        const long long n = el.conn_all[8 * e + l];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            u[d] = nd.u[3 * n + d];
+            x[d] = nd.pos[3 * n + d] + u[d];
+            gk[d] = G[(SC_GRAD + 3 * l + d) * S + i];
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) ak[a] = G[(SC_GAMMA + 4 * l + a) * S + i];
+#pragma unroll
+        for (int c = 0; c < 12; ++c) {
+            h0[c] = G[(SC_H + h_index(l, c)) * S + i];
+            if (l < 4) h1[c] = G[(SC_H + h_index(row1, c)) * S + i];
+        }
+        vol = G[SC_VOL * S + i];
+        youngs = el.sc_mat[2 * i];
+        poisson = el.sc_mat[2 * i + 1];
+    }
+    // node k's x, dN/dX, u and gamma at sh[13 k]
+    double* mine = sh + 13 * l;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        mine[d] = x[d];
+        mine[3 + d] = gk[d];
+        mine[6 + d] = u[d];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) mine[9 + a] = ak[a];
+    __syncwarp();
+    // components 0-8: F[3 a + b]; 9-20: q[3 a + d]
+    double comp[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int c = l + 8 * r;
+        const int p = c < 9 ? c / 3 : 6 + (c - 9) % 3, q = c < 9 ? 3 + c % 3 : 9 + (c < 21 ? (c - 9) / 3 : 0);
+        double s = sh[p] * sh[q];
+        if (c < 9) s = 0.0 + s;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s = s + sh[13 * k + p] * sh[13 * k + q];
+        comp[r] = s;
+    }
+    __syncwarp();  // every lane has read the nodes
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        if (l + 8 * r < 21) sh[l + 8 * r] = comp[r];
+    __syncwarp();
+    double f[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) f[k] = sh[k];
+    const double det = det3d(f);
+    if (live && det <= 0.0) {
+        if (l == 0) {
+            el.eroded_all[e] = 1;
+            atomicAdd(reinterpret_cast<unsigned long long*>(&ctls[slot].eroded_step), 1ull);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) out[3 * l + d] = 0.0;
+        live = false;
+    }
+    double tau[9];
+    hencky_elastic_oct(youngs, poisson, f, tau, l);
+    // inverse of f (inv3d), entry l on lane l, entry 8 on every lane
+    double fi[2];
+    {
+        // entry = sign (a[i0] a[i1] - a[i2] a[i3]) / det
+        const uint32_t idx[9] = {0x4875, 0x1872, 0x1542, 0x3865, 0x0862, 0x0532, 0x3764, 0x0761, 0x0431};
+        uint32_t t = idx[0];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) t = l == k ? idx[k] : t;
+        const double m = sh[t >> 12] * sh[(t >> 8) & 15] - sh[(t >> 4) & 15] * sh[t & 15];
+        fi[0] = ((l & 1) ? -m : m) / det;
+        fi[1] = (f[0] * f[4] - f[3] * f[1]) / det;
+    }
+    double* finv = sh + 24;  // 9
+    double* rr = sh + 33;    // 12
+    finv[l] = fi[0];
+    if (l == 0) finv[8] = fi[1];
+    {
+        double q[12];
+#pragma unroll
+        for (int c = 0; c < 12; ++c) q[c] = sh[9 + c];
+        double t0 = h0[0] * q[0], t1 = h1[0] * q[0];
+#pragma unroll
+        for (int c = 1; c < 12; ++c) {
+            t0 = t0 + h0[c] * q[c];
+            t1 = t1 + h1[c] * q[c];
+        }
+        rr[l] = t0;
+        if (l < 4) rr[row1] = t1;
+    }
+    __syncwarp();
+    double m[9];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            double t = tau[3 * a] * finv[3 * b];
+            t = t + tau[3 * a + 1] * finv[3 * b + 1];
+            t = t + tau[3 * a + 2] * finv[3 * b + 2];
+            m[3 * a + b] = t * vol;
+        }
+    if (live)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            double o = m[3 * d] * gk[0];
+            o = o + m[3 * d + 1] * gk[1];
+            o = o + m[3 * d + 2] * gk[2];
+            double t = rr[d] * ak[0];
+#pragma unroll
+            for (int a = 1; a < 4; ++a) t = t + rr[3 * a + d] * ak[a];
+            out[3 * l + d] = o + t;
+        }
+    __syncwarp();  // sh is free again
+}
+
 __global__ void __launch_bounds__(SC_TPB) k_forces_scalar(ElementArrays el, NodeArrays nd, Control* ctls, int respect_done) {
     FOR_ACTIVE(el.act_sc, el.n_sc, 1, g) {
         int lane;
@@ -806,6 +959,22 @@ __global__ void __launch_bounds__(SC_TPB) k_forces_scalar(ElementArrays el, Node
         // a run lists the elastic elements with a free node; drop-in calls take them all
         scalar_force_body<false>(el, nd, ctls, ctls, respect_done, el.sc_list ? (t < el.n_sc ? (long long)el.sc_list[t] : el.sc_count) : t);
     }
+}
+
+// Both kinds of a small mesh in one launch: blocks [0, hc_blocks) take 64
+// honeycomb elements each, the rest 8 elastic ones on eight lanes each. Small
+// blocks spread a few elements over the SMs, and the elastic elements (a
+// road's 360 took a launch of their own behind the others) run beside them: a
+// force call on 1290 + 264 elements takes 7.4 us, 12.3 us in three launches.
+constexpr int SMALL_TPB = 64;
+__global__ void __launch_bounds__(SMALL_TPB) k_forces_small(ElementArrays el, NodeArrays nd, Control* ctls, int respect_done, int hc_blocks) {
+    __shared__ double sh[SMALL_TPB / 8][OCT_SHARED];
+    if ((int)blockIdx.x < hc_blocks) {
+        forces_body(el, nd, ctls, ctls, respect_done, (long long)blockIdx.x * SMALL_TPB + threadIdx.x);
+        return;
+    }
+    const long long i = (long long)(blockIdx.x - hc_blocks) * (SMALL_TPB / 8) + threadIdx.x / 8;
+    scalar_force_oct(el, nd, ctls, ctls, respect_done, i < el.n_sc ? i : -1, sh[threadIdx.x / 8]);
 }
 
 // The elastic elements' corner forces on node n, component d, added to f in
@@ -2225,18 +2394,48 @@ __global__ void k_node_cn(const uint32_t* __restrict__ cnode, long long i0, long
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
+// Asked once per device (the queries take some 0.2 ms).
 int resident_blocks(int device, int n_sms) {
-    int coop = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_steps<RES_SMALL>, RES_SMALL, 0) != cudaSuccess || per_sm < 1) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_steps<RES_LARGE>, RES_LARGE, 0) != cudaSuccess || per_sm < 1) return 0;
-    return n_sms;
+    constexpr int DEVICES = 64;
+    static std::atomic<int> known[DEVICES];  // 0 not asked, 1 no, 2 yes
+    if (device >= 0 && device < DEVICES && known[device].load()) return known[device].load() == 2 ? n_sms : 0;
+    const auto ask = [&] {
+        int coop = 0, per_sm = 0;
+        if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return false;
+        const auto fits = [&](auto kernel, int tpb, size_t bytes) {
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess &&
+                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tpb, bytes) == cudaSuccess && per_sm >= 1;
+        };
+        const size_t oct = sizeof(double) * OCT_SHARED / 8;  // per thread
+        return fits(k_steps<RES_SMALL, false>, RES_SMALL, 0) && fits(k_steps<RES_LARGE, false>, RES_LARGE, 0) &&
+               fits(k_steps<RES_SMALL, true>, RES_SMALL, oct * RES_SMALL) && fits(k_steps<RES_LARGE, true>, RES_LARGE, oct * RES_LARGE);
+    };
+    const bool yes = ask();
+    if (device >= 0 && device < DEVICES) known[device].store(yes ? 2 : 1);
+    return yes ? n_sms : 0;
 }
 cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks) {
-    void* args[] = {const_cast<ResidentArgs*>(&a)};
-    if (a.el.n_hc > 32 * (RES_SMALL / 32) * (long long)blocks)
-        return cudaLaunchCooperativeKernel(k_steps<RES_LARGE>, dim3((unsigned)blocks), dim3(RES_LARGE), args, 0, s);
-    return cudaLaunchCooperativeKernel(k_steps<RES_SMALL>, dim3((unsigned)blocks), dim3(RES_SMALL), args, 0, s);
+    // Elastic elements on eight lanes each while all their lanes fit the grid
+    // beside the honeycomb elements' threads.
+    ResidentArgs b = a;
+    const long long small = (long long)RES_SMALL * blocks, large = (long long)RES_LARGE * blocks;
+    const long long wide = a.el.n_hc + 8 * a.el.n_sc;
+    b.sc_oct = a.el.n_sc > 0 && wide <= large ? 1 : 0;
+    const bool big = b.sc_oct ? wide > small : a.el.n_hc > small;
+    void* args[] = {&b};
+    const size_t smem = b.sc_oct ? sizeof(double) * OCT_SHARED * (big ? RES_LARGE : RES_SMALL) / 8 : 0;
+    const dim3 grid((unsigned)blocks), tpb(big ? RES_LARGE : RES_SMALL);
+    if (smem > 0) {  // set anew each time: a device reset between two contexts drops it
+        const cudaError_t e = big ? cudaFuncSetAttribute(k_steps<RES_LARGE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                                  : cudaFuncSetAttribute(k_steps<RES_SMALL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    if (a.el.n_sc > 0) {
+        if (big) return cudaLaunchCooperativeKernel(k_steps<RES_LARGE, true>, grid, tpb, args, smem, s);
+        return cudaLaunchCooperativeKernel(k_steps<RES_SMALL, true>, grid, tpb, args, smem, s);
+    }
+    if (big) return cudaLaunchCooperativeKernel(k_steps<RES_LARGE, false>, grid, tpb, args, smem, s);
+    return cudaLaunchCooperativeKernel(k_steps<RES_SMALL, false>, grid, tpb, args, smem, s);
 }
 void launch_node_cn(cudaStream_t s, const uint32_t* cnode, long long i0, long long i1, uint32_t* node_cn) {
     if (i1 > i0) k_node_cn<<<(unsigned)blocks_for(i1 - i0, TPB), TPB, 0, s>>>(cnode, i0, i1, node_cn);
@@ -2331,6 +2530,11 @@ void launch_init_state(cudaStream_t s, long long h_begin, long long n_hc, long l
     if (n_hc <= h_begin) return;
     k_init_state<<<(unsigned)blocks_for(n_hc - h_begin, TPB), TPB, 0, s>>>(h_begin, n_hc, stride, state);
 }
+// A mesh that k_forces_small takes: every element (no active lists), at most
+// 128 threads per SM of either kind, where a lone wave's latency is all there is.
+bool small_forces(const ElementArrays& el) {
+    return !el.act_hc.list && !el.sc_list && el.n_sc == el.sc_count && el.n_hc <= 148 * 128 && 8 * el.n_sc <= 148 * 128;
+}
 void launch_forces(cudaStream_t s, const ElementArrays& el, const NodeArrays& nd, Control* ctls, int respect_done, int n_sms,
                    int schedule, unsigned* queue) {
     // Schedule 0, persistent: one wave of FORCES_MINB blocks per SM taking
@@ -2339,6 +2543,11 @@ void launch_forces(cudaStream_t s, const ElementArrays& el, const NodeArrays& nd
     // contact pass) gets SMs while the kernel runs. Schedule 2 (3): the
     // persistent wave on all but 8 (16) SMs, which stay free for the side
     // streams' search. Without a queue, the persistent waves stride instead.
+    if (small_forces(el)) {
+        const unsigned hb = (unsigned)blocks_for(el.n_hc, SMALL_TPB), sb = (unsigned)blocks_for(8 * el.n_sc, SMALL_TPB);
+        if (hb + sb > 0) k_forces_small<<<hb + sb, SMALL_TPB, 0, s>>>(el, nd, ctls, respect_done, (int)hb);
+        return;
+    }
     const int free_sms = schedule == 2 ? 8 : schedule == 3 ? 16 : 0;
     long long cap = (long long)(n_sms > 2 * free_sms ? n_sms - free_sms : n_sms) * FORCES_MINB;
     if (schedule == 1) cap = GRID_CAP * 4;
@@ -2348,7 +2557,10 @@ void launch_forces(cudaStream_t s, const ElementArrays& el, const NodeArrays& nd
     if (el.n_sc > 0)
         k_forces_scalar<<<active_grid(el.n_sc, 1, SC_TPB, GRID_CAP), SC_TPB, 0, s>>>(el, nd, ctls, respect_done);
 }
-int forces_launches(const ElementArrays& el) { return (el.n_hc > 0 ? 1 : 0) + (el.n_sc > 0 ? 1 : 0); }
+int forces_launches(const ElementArrays& el) {
+    if (small_forces(el)) return el.n_hc + el.n_sc > 0 ? 1 : 0;
+    return (el.n_hc > 0 ? 1 : 0) + (el.n_sc > 0 ? 1 : 0);
+}
 void launch_gather(cudaStream_t s, const ElementArrays& el, const NodeArrays& nd, double* f_out) {
     k_gather<<<(unsigned)blocks_for(nd.n, TPB), TPB, 0, s>>>(el, nd, f_out);
 }

@@ -447,6 +447,7 @@ struct ResidentArgs {
     int n_steps;
     int adaptive, check_steps, any_separation, hist_on;
     long long n_slaves;
+    int sc_oct;           // elastic elements on eight lanes each (set by the launcher)
     const int* lists;     // active chunk lists (ab.lists), or null: every chunk of every space
     long long space_off[ACTIVE_SPACES];
     long long space_n[ACTIVE_SPACES];

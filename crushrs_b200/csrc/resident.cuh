@@ -221,6 +221,7 @@ __device__ __forceinline__ void resident_gather_half(const ContactArrays& ca, co
 
 // A node's full update: full_body's arithmetic for its three components, its
 // incidence read once.
+template <bool ELASTIC>
 __device__ __forceinline__ void resident_full(const ElementArrays& el, const NodeArrays& nd, const ControlView* view, long long n) {
     if (n >= nd.n) return;
     const ControlView* ctl = view + nd.node_slot[n];
@@ -249,7 +250,7 @@ __device__ __forceinline__ void resident_full(const ElementArrays& el, const Nod
 #pragma unroll
         for (int d = 0; d < 3; ++d) f[d] = gather_component(nd, el.corner, n, d);
     }
-    if (el.n_sc > 0)
+    if (ELASTIC)
 #pragma unroll
         for (int d = 0; d < 3; ++d) f[d] = add_scalar_corners(el, nd, n, d, f[d]);
     if (ctl->done) return;
@@ -263,7 +264,128 @@ __device__ __forceinline__ void resident_full(const ElementArrays& el, const Nod
     }
 }
 
-template <int RES_TPB>
+// ELASTIC: the context has elastic elements with a free node; without, their
+// code stays out of the kernel.
+// A static-grid entry by RES_ST_LANES lanes: nothing outside the union of the
+// fixed faces' key boxes, else the faces of its point's bucket, smallest first
+// (contact_slave_body's static part). Every lane of the warp calls; the face, or
+// -1, in the first lane of the entry.
+__device__ __forceinline__ int resident_static(const ContactArrays& ca, const NodeArrays& nd, const ControlView* view, long long s, bool live,
+                                               int lane, double* sd_out) {
+    int best = INT_MAX;
+    double best_sd = 0.0, sd;
+    if (live) {
+        const int c = ca.slave_contact[s];
+        const long long n = ca.slaves[s];
+        const double p[3] = {nd.pos[3 * n] + nd.u[3 * n], nd.pos[3 * n + 1] + nd.u[3 * n + 1], nd.pos[3 * n + 2] + nd.u[3 * n + 2]};
+        const double* box = ca.st_box + 6 * c;
+        live = !view[ca.contact_slot[c]].done;
+        if (live && p[0] >= box[0] && p[0] <= box[3] && p[1] >= box[1] && p[1] <= box[4] && p[2] >= box[2] && p[2] <= box[5]) {
+            const double md = ca.max_distance[c];
+            const FaceGeo* geo = ca.geo + ca.face_off[c];
+            const long long st0 = ca.st_tab_off[c];
+            const long long bk = st0 + (point_cell_hash(p, ca.cell[c], 0) & (unsigned)(ca.st_tab_off[c + 1] - st0 - 1));
+            const uint32_t e0 = ca.st_off[bk + c], e1 = ca.st_off[bk + c + 1];
+            for (uint32_t k = e0 + lane; k < e1; k += RES_ST_LANES) {  // ascending faces: a lane's first hit is its smallest
+                const int f = ca.st_entries[k];
+                if (face_hit(geo[f], p, md, &sd)) {
+                    best = f;
+                    best_sd = sd;
+                    break;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int off = RES_ST_LANES / 2; off > 0; off >>= 1) {
+        const int ob = __shfl_down_sync(0xffffffffu, best, off, RES_ST_LANES);
+        const double osd = __shfl_down_sync(0xffffffffu, best_sd, off, RES_ST_LANES);
+        if (ob < best) {
+            best = ob;
+            best_sd = osd;
+        }
+    }
+    if (!live || lane != 0) return -1;
+    if (best == INT_MAX) {
+        ca.hit[s] = -1;
+        return -1;
+    }
+    ca.hit[s] = best;
+    ca.hit_sd[s] = best_sd;
+    *sd_out = best_sd;
+    return best;
+}
+// A dynamic-grid entry (or one of a contact without any grid) by a warp:
+// contact_slave_body's dynamic part with one list of candidates, so that a
+// single narrow test serves all of them. Every lane calls; the face, or -1, in
+// lane 0. (A step of the 20,048-element T-bone takes 29 us, 31 us with the
+// buckets of the levels scanned one after the other.)
+__device__ __forceinline__ int resident_grid(const ContactArrays& ca, const NodeArrays& nd, const ControlView* view, long long s, bool live,
+                                             int l, double* sd_out) {
+    int best = INT_MAX;
+    double best_sd = 0.0;
+    bool reset_big = false;
+    if (live) {
+        const int c = ca.slave_contact[s];
+        const long long n = ca.slaves[s];
+        const int tab = ca.tab_off[c], tab1 = ca.tab_off[c + 1];
+        reset_big = l == 0 && tab1 > tab;
+        const double p[3] = {nd.pos[3 * n] + nd.u[3 * n], nd.pos[3 * n + 1] + nd.u[3 * n + 1], nd.pos[3 * n + 2] + nd.u[3 * n + 2]};
+        const double md = ca.max_distance[c];
+        const long long fb = ca.face_off[c];
+        const FaceGeo* geo = ca.geo + fb;
+        live = !view[ca.contact_slot[c]].done;
+        // the candidates: the smallest big face that hit (one more for lane 0),
+        // then the point's bucket of every level in use, or all the faces
+        const int big = live && tab1 > tab ? ca.big_best[s] : BIG_NONE;
+        const int used = tab1 > tab ? ca.levels_used[c] : 0;
+        const unsigned mask = (unsigned)(tab1 - tab - 1);
+        unsigned e0[GRID_LEVELS] = {0u, 0u};
+        int cnt[GRID_LEVELS] = {0, 0};
+        if (live && tab1 > tab) {
+            double cs = ca.cell[c];
+#pragma unroll
+            for (int level = 0; level < GRID_LEVELS; ++level, cs *= 4.0)
+                if (used & (1 << level)) {
+                    const int b = tab + (int)(point_cell_hash(p, cs, level) & mask);
+                    e0[level] = ca.boff[b];
+                    cnt[level] = ca.blen[b];
+                }
+        }
+        const int lead = big != BIG_NONE ? 1 : 0;
+        const int total = !live ? 0 : tab1 > tab ? lead + cnt[0] + cnt[1] : (int)(ca.face_off[c + 1] - fb);
+        for (int k = l; k < total; k += RES_GRID_LANES) {
+            int f = k;
+            if (tab1 > tab) f = k < lead ? big : k < lead + cnt[0] ? ca.entries[e0[0] + k - lead] : ca.entries[e0[1] + k - lead - cnt[0]];
+            double sd;
+            if (f < best && face_hit(geo[f], p, md, &sd)) {
+                best = f;
+                best_sd = sd;
+            }
+        }
+    }
+#pragma unroll
+    for (int off = RES_GRID_LANES / 2; off > 0; off >>= 1) {
+        const int ob = __shfl_down_sync(0xffffffffu, best, off, RES_GRID_LANES);
+        const double osd = __shfl_down_sync(0xffffffffu, best_sd, off, RES_GRID_LANES);
+        if (ob < best) {
+            best = ob;
+            best_sd = osd;
+        }
+    }
+    static_assert(GRID_LEVELS == 2, "two levels' buckets");
+    if (reset_big) ca.big_best[s] = BIG_NONE;
+    if (!live || l != 0) return -1;
+    if (best == INT_MAX) {
+        ca.hit[s] = -1;
+        return -1;
+    }
+    ca.hit[s] = best;
+    ca.hit_sd[s] = best_sd;
+    *sd_out = best_sd;
+    return best;
+}
+template <int RES_TPB, bool ELASTIC>
 __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ ResidentArgs A) {
     __shared__ HeavyShared heavy;
     __shared__ FaceGeo big_face;
@@ -271,6 +393,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
     __shared__ int s_state, s_chunks[ACTIVE_SPACES];
     __shared__ uint8_t s_cand[RES_TPB / 32][BRUTE_MAX_FACES + 1];
     __shared__ ControlView view[RESIDENT_MAX_SLOTS];
+    extern __shared__ double oct_shared[];  // OCT_SHARED per eight threads, when elastic elements take eight lanes
     constexpr int RES_WARPS = RES_TPB / 32;
     static_assert(RES_TPB >= HEAVY_TPB && VEH_TPB == HEAVY_TPB && sizeof(heavy.sf) >= 2 * sizeof(double) * VEH_TPB, "block sums");
     const bool summing = threadIdx.x < HEAVY_TPB;  // the threads of the block-wide sums
@@ -423,7 +546,14 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             int l;
             forces_body(el, nd, ctls, view, 1, entity(0, t, 1, &l));
         });
-        if (el.n_sc > 0)
+        if (ELASTIC && A.sc_oct)
+            deal(tasks(8, 8), [&](int t) {
+                int l;
+                const long long k = entity(8, t, 8, &l);
+                scalar_force_oct(el, nd, ctls, view, 1, k < el.n_sc ? (long long)el.sc_list[k] : -1,
+                                 oct_shared + OCT_SHARED * (threadIdx.x / 8));
+            });
+        else if (ELASTIC)
             deal(tasks(8, 1), [&](int t) {
                 int l;
                 const long long k = entity(8, t, 1, &l);
@@ -457,7 +587,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             const bool live = e < ca.n_st_slaves;
             const long long s = live ? (long long)ca.st_slaves[e] : 0;
             double sd = 0.0;
-            const int best = contact_slave_body<RES_ST_LANES>(cn, nd, view, 0, ca.n_contacts, 1, 0.0, nullptr, s, live, l, &sd);
+            const int best = resident_static(cn, nd, view, s, live, l, &sd);
             if (plain) resident_emit<RES_ST_LANES>(cn, view, nd.mass, s, best, sd, l);
         });
         if (check_next)
@@ -467,7 +597,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             });
         deal(tasks(2, 1), [&](int t) {
             int l;
-            resident_full(el, nd, view, entity(2, t, 1, &l));
+            resident_full<ELASTIC>(el, nd, view, entity(2, t, 1, &l));
         });
         if ((step + 1) % 20 == 0)
             deal(tasks(2, 1), [&](int t) {
@@ -494,7 +624,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                 const bool live = e < ca.n_grid_slaves;
                 const long long s = live ? (long long)ca.grid_slaves[e] : 0;
                 double sd = 0.0;
-                const int best = contact_slave_body<RES_GRID_LANES>(cn, nd, view, 0, ca.n_contacts, 1, 0.0, nullptr, s, live, l, &sd);
+                const int best = resident_grid(cn, nd, view, s, live, l, &sd);
                 if (plain) resident_emit<RES_GRID_LANES>(cn, view, nd.mass, s, best, sd, l);
             });
         }
