@@ -521,6 +521,7 @@ struct crush_ctx {
     std::vector<int> hist_steps;                 // per slot: history_steps, 0 = off
     std::vector<long long> hist_max;             // per slot: records kept
     std::vector<std::vector<HistAccel>> hist_acc;
+    std::vector<std::vector<std::vector<uint32_t>>> hist_parts;  // per slot that has recorded: its parts' nodes, ascending
     HistoryArrays hist{};
     bool hist_on = false;
     bool hist_ran = false;                       // a run began since the configuration
@@ -2532,24 +2533,32 @@ int rebuild_history(crush_ctx* c) {
     std::vector<int> on(c->n_slots), pu_slot_off(c->n_slots + 1, 0), an_off(c->n_slots + 1, 0), pu_slot, an_frame;
     std::vector<long long> smax(c->n_slots, 0);
     std::vector<uint32_t> pu_off(1, 0), pu_nodes, an_node, fr_nodes;
+    c->hist_parts.resize(c->n_slots);
     for (int k = 0; k < c->n_slots; ++k) {
         const Slot& sl = c->slots[k];
         on[k] = c->hist_steps[k] > 0;
         smax[k] = on[k] ? c->hist_max[k] : 0;
         if (on[k]) {
-            // part_nodes (src/mesh.rs:74-82): ascending nodes of each part's elements
-            std::vector<int32_t> part(sl.n_elems);
-            std::vector<uint32_t> conn(8 * sl.n_elems);
-            CK(cudaMemcpy(part.data(), c->part + sl.elem0, sizeof(int32_t) * sl.n_elems, cudaMemcpyDeviceToHost));
-            CK(cudaMemcpy(conn.data(), c->conn_all + 8 * sl.elem0, sizeof(uint32_t) * 8 * sl.n_elems, cudaMemcpyDeviceToHost));
-            std::vector<std::vector<uint32_t>> nodes(sl.n_parts);
-            for (long long e = 0; e < sl.n_elems; ++e) {
-                const int p = part[e] - sl.part0;
-                if (p >= 0 && p < sl.n_parts) nodes[p].insert(nodes[p].end(), conn.begin() + 8 * e, conn.begin() + 8 * e + 8);
+            // part_nodes (src/mesh.rs:74-82): ascending nodes of each part's
+            // elements, built once per slot (every configuration call comes
+            // here, for all the slots configured before it)
+            std::vector<std::vector<uint32_t>>& nodes = c->hist_parts[k];
+            if (nodes.empty() && sl.n_parts > 0) {
+                std::vector<int32_t> part(sl.n_elems);
+                std::vector<uint32_t> conn(8 * sl.n_elems);
+                CK(cudaMemcpy(part.data(), c->part + sl.elem0, sizeof(int32_t) * sl.n_elems, cudaMemcpyDeviceToHost));
+                CK(cudaMemcpy(conn.data(), c->conn_all + 8 * sl.elem0, sizeof(uint32_t) * 8 * sl.n_elems, cudaMemcpyDeviceToHost));
+                nodes.resize(sl.n_parts);
+                for (long long e = 0; e < sl.n_elems; ++e) {
+                    const int p = part[e] - sl.part0;
+                    if (p >= 0 && p < sl.n_parts) nodes[p].insert(nodes[p].end(), conn.begin() + 8 * e, conn.begin() + 8 * e + 8);
+                }
+                for (auto& v : nodes) {
+                    std::sort(v.begin(), v.end());
+                    v.erase(std::unique(v.begin(), v.end()), v.end());
+                }
             }
-            for (auto& v : nodes) {
-                std::sort(v.begin(), v.end());
-                v.erase(std::unique(v.begin(), v.end()), v.end());
+            for (const auto& v : nodes) {
                 pu_nodes.insert(pu_nodes.end(), v.begin(), v.end());
                 pu_off.push_back((uint32_t)pu_nodes.size());
                 pu_slot.push_back(k);
@@ -3641,12 +3650,15 @@ int crush_history_get(crush_ctx* c, int slot, double* time, int64_t* step, crush
         for (long long k = 0; k < kept; ++k) step[k] = s[k];
     }
     if (parts && n_parts > 0) {
-        std::vector<double> buf((size_t)n_parts * stride * HIST_PART_VALUES);
-        CK(cudaMemcpy(buf.data(), h.part_rec + pu_off[slot] * stride * HIST_PART_VALUES, sizeof(double) * buf.size(),
-                      cudaMemcpyDeviceToHost));
+        // the kept records of every part, not the room for max_records (18
+        // probes with room for 20,000 records that kept 1030: 52 ms, now 12 ms)
+        const size_t row = sizeof(double) * HIST_PART_VALUES;
+        std::vector<double> buf((size_t)n_parts * kept * HIST_PART_VALUES);
+        CK(cudaMemcpy2D(buf.data(), row * kept, h.part_rec + pu_off[slot] * stride * HIST_PART_VALUES, row * stride, row * kept, n_parts,
+                        cudaMemcpyDeviceToHost));
         for (long long r = 0; r < kept; ++r)
             for (int p = 0; p < n_parts; ++p) {
-                const double* v = &buf[((size_t)p * stride + r) * HIST_PART_VALUES];
+                const double* v = &buf[((size_t)p * kept + r) * HIST_PART_VALUES];
                 crush_part_state& o = parts[r * n_parts + p];
                 o.mass = v[0];
                 for (int d = 0; d < 3; ++d) {
@@ -3658,15 +3670,16 @@ int crush_history_get(crush_ctx* c, int slot, double* time, int64_t* step, crush
             }
     }
     if (samples && n_nodes > 0) {
-        std::vector<double> buf((size_t)n_nodes * stride * HIST_NODE_VALUES);
-        CK(cudaMemcpy(buf.data(), h.node_rec + an_off[slot] * stride * HIST_NODE_VALUES, sizeof(double) * buf.size(),
-                      cudaMemcpyDeviceToHost));
+        const size_t row = sizeof(double) * HIST_NODE_VALUES;
+        std::vector<double> buf((size_t)n_nodes * kept * HIST_NODE_VALUES);
+        CK(cudaMemcpy2D(buf.data(), row * kept, h.node_rec + an_off[slot] * stride * HIST_NODE_VALUES, row * stride, row * kept, n_nodes,
+                        cudaMemcpyDeviceToHost));
         std::vector<std::pair<int, uint32_t>> who;  // (accelerometer, node) of each sampled node
         for (size_t k = 0; k < c->hist_acc[slot].size(); ++k)
             for (uint32_t n : c->hist_acc[slot][k].nodes) who.push_back({(int)k, n});
         for (long long r = 0; r < kept; ++r)
             for (long long j = 0; j < n_nodes; ++j) {
-                const double* v = &buf[((size_t)j * stride + r) * HIST_NODE_VALUES];
+                const double* v = &buf[((size_t)j * kept + r) * HIST_NODE_VALUES];
                 crush_node_sample& o = samples[r * n_nodes + j];
                 o.accelerometer = who[j].first;
                 o.node = who[j].second;
