@@ -1775,7 +1775,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         CK(cudaMemcpyAsync(c->voff_d, &zero, sizeof(long long), cudaMemcpyHostToDevice, c->stream));
         CK(cudaStreamSynchronize(c->stream));  // the zero above is a stack value
         // active chunk tables: every space's chunks at its full room
-        const long long sizes[ACTIVE_SPACES] = {EC, EC, NC, SC, CNC, FC, SC, SC, QC};
+        const long long sizes[ACTIVE_SPACES] = {EC, EC, NC, SC, CNC, FC, SC, SC, QC, SC};
         c->space_off_h.assign(ACTIVE_SPACES + 1, 0);
         for (int sp = 0; sp < ACTIVE_SPACES; ++sp) c->space_off_h[sp + 1] = c->space_off_h[sp] + (sizes[sp] + CHUNK - 1) / CHUNK;
         const long long nch = c->space_off_h[ACTIVE_SPACES];
@@ -1927,9 +1927,10 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     // ---- active chunk tables: the slot range of every chunk the new entities touch ----
     {
         const long long ends[ACTIVE_SPACES] = {c->n_hc, c->n_all, c->n_nodes, ca.n_grid_slaves, ca.n_cnodes, ca.n_dyn_faces,
-                                               c->n_slaves, ca.n_st_slaves, c->n_sc_free};
+                                               c->n_slaves, ca.n_st_slaves, c->n_sc_free, ca.n_brute_entries};
         const long long begins[ACTIVE_SPACES] = {H0, E0, N0, ca.n_grid_slaves - (long long)gslaves.size(), base[0].cnode, base[0].dyn,
-                                                 SB, ca.n_st_slaves - (long long)stslaves.size(), QF0};
+                                                 SB, ca.n_st_slaves - (long long)stslaves.size(), QF0,
+                                                 ca.n_brute_entries - (long long)bents.size()};
         auto slot_of = [&](int sp, long long i) -> int {
             switch (sp) {
                 case 0: return (int)cm.elem_slot[hc_model[i - H0] - E0];
@@ -1940,7 +1941,8 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
                 case 5: return contact_slot[face_contact[dyn_faces[i - base[0].dyn] - FB] - K0];
                 case 6: return contact_slot[slave_contact[i - SB] - K0];
                 case 7: return contact_slot[slave_contact[stslaves[i - begins[7]] - SB] - K0];
-                default: return (int)cm.elem_slot[sc_model[sc_list[i - QF0] - Q0] - E0];
+                case 8: return (int)cm.elem_slot[sc_model[sc_list[i - QF0] - Q0] - E0];
+                default: return bents[i - begins[9]].slot;
             }
         };
         for (int sp = 0; sp < ACTIVE_SPACES; ++sp) {
@@ -2912,11 +2914,27 @@ int schedule_trial(crush_ctx* c) {
 constexpr long long RESIDENT_MAX_ELEMENTS = 160000;
 constexpr long long RESIDENT_MAX_STEPS = 1000;  // steps of one launch
 
+// Honeycomb elements of the slots that the last read of the done flags left
+// running, and the first of those slots.
+long long busy_elements(const crush_ctx* c, int* first) {
+    long long n = 0;
+    int f = -1;
+    for (int k = 0; k < c->n_slots; ++k)
+        if (k >= (int)c->done_h.size() || !c->done_h[k]) {
+            n += c->slots[k].n_hc;
+            if (f < 0) f = k;
+        }
+    if (first) *first = f;
+    return n;
+}
+
 // Whether the context's steps run in the resident kernel: small, on the
 // automatic schedule, with nothing between the steps but what that kernel does.
+// The size is that of the crashes not known to be done (a serving context keeps
+// the finished ones; the kernel visits the others' chunks).
 bool resident(const crush_ctx* c) {
     return c->res_blocks > 0 && !c->tuning_fixed && !c->profiling && !c->ca.exhaustive && !c->frames_on &&
-           c->n_hc + c->n_sc_free <= RESIDENT_MAX_ELEMENTS && c->n_slots <= RESIDENT_MAX_SLOTS;
+           busy_elements(c, nullptr) + c->n_sc_free <= RESIDENT_MAX_ELEMENTS && c->n_slots <= RESIDENT_MAX_SLOTS;
 }
 
 int resident_steps(crush_ctx* c, long long n) {
@@ -2941,13 +2959,18 @@ int resident_steps(crush_ctx* c, long long n) {
     a.any_separation = c->any_separation ? 1 : 0;
     a.hist_on = c->hist_on ? 1 : 0;
     a.n_slaves = c->n_slaves;
+    int first = -1;
+    a.n_busy = busy_elements(c, &first);
+    a.contact0 = first < 0 ? 0 : c->slots[first].contact0;
     // One crash: every chunk, until it is done; more: those of running crashes.
     a.lists = c->n_slots > 1 ? c->ab.lists : nullptr;
     const long long ns[ACTIVE_SPACES] = {c->n_hc, c->n_all, c->n_nodes, c->ca.n_grid_slaves, c->ca.n_cnodes, c->ca.n_dyn_faces,
-                                         c->n_slaves, c->ca.n_st_slaves, c->n_sc_free};
+                                         c->n_slaves, c->ca.n_st_slaves, c->n_sc_free, c->ca.n_brute_entries};
+    a.chunk_off[0] = 0;
     for (int k = 0; k < ACTIVE_SPACES; ++k) {
         a.space_off[k] = c->space_off_h[k];
         a.space_n[k] = ns[k];
+        a.chunk_off[k + 1] = a.chunk_off[k] + (int)((ns[k] + CHUNK - 1) / CHUNK);
     }
     CK(cudaMemsetAsync(c->res_sync, 0, sizeof(ResidentSync), c->stream));
     CK(launch_resident(c->stream, a, c->res_blocks));

@@ -2406,9 +2406,10 @@ int resident_blocks(int device, int n_sms) {
             return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess &&
                    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tpb, bytes) == cudaSuccess && per_sm >= 1;
         };
-        const size_t oct = sizeof(double) * OCT_SHARED / 8;  // per thread
-        return fits(k_steps<RES_SMALL, false>, RES_SMALL, 0) && fits(k_steps<RES_LARGE, false>, RES_LARGE, 0) &&
-               fits(k_steps<RES_SMALL, true>, RES_SMALL, oct * RES_SMALL) && fits(k_steps<RES_LARGE, true>, RES_LARGE, oct * RES_LARGE);
+        const size_t oct = sizeof(double) * OCT_SHARED / 8, views = sizeof(ControlView) * RESIDENT_MAX_SLOTS;  // oct: per thread
+        return fits(k_steps<RES_SMALL, false>, RES_SMALL, views) && fits(k_steps<RES_LARGE, false>, RES_LARGE, views) &&
+               fits(k_steps<RES_SMALL, true>, RES_SMALL, views + oct * RES_SMALL) &&
+               fits(k_steps<RES_LARGE, true>, RES_LARGE, views + oct * RES_LARGE);
     };
     const bool yes = ask();
     if (device >= 0 && device < DEVICES) known[device].store(yes ? 2 : 1);
@@ -2419,23 +2420,20 @@ cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks) {
     // beside the honeycomb elements' threads.
     ResidentArgs b = a;
     const long long small = (long long)RES_SMALL * blocks, large = (long long)RES_LARGE * blocks;
-    const long long wide = a.el.n_hc + 8 * a.el.n_sc;
+    const long long wide = a.n_busy + 8 * a.el.n_sc;
     b.sc_oct = a.el.n_sc > 0 && wide <= large ? 1 : 0;
-    const bool big = b.sc_oct ? wide > small : a.el.n_hc > small;
+    const bool big = b.sc_oct ? wide > small : a.n_busy > small;
     void* args[] = {&b};
-    const size_t smem = b.sc_oct ? sizeof(double) * OCT_SHARED * (big ? RES_LARGE : RES_SMALL) / 8 : 0;
+    const size_t smem = (b.sc_oct ? sizeof(double) * OCT_SHARED * (big ? RES_LARGE : RES_SMALL) / 8 : 0) +
+                        sizeof(ControlView) * (size_t)a.ca[0].n_slots;
     const dim3 grid((unsigned)blocks), tpb(big ? RES_LARGE : RES_SMALL);
-    if (smem > 0) {  // set anew each time: a device reset between two contexts drops it
-        const cudaError_t e = big ? cudaFuncSetAttribute(k_steps<RES_LARGE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                                  : cudaFuncSetAttribute(k_steps<RES_SMALL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const void* kernel = a.el.n_sc > 0 ? (big ? (const void*)k_steps<RES_LARGE, true> : (const void*)k_steps<RES_SMALL, true>)
+                                       : (big ? (const void*)k_steps<RES_LARGE, false> : (const void*)k_steps<RES_SMALL, false>);
+    if (smem > 12 * 1024) {  // past the default beside the static part; set anew each time: a device reset between two contexts drops it
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    if (a.el.n_sc > 0) {
-        if (big) return cudaLaunchCooperativeKernel(k_steps<RES_LARGE, true>, grid, tpb, args, smem, s);
-        return cudaLaunchCooperativeKernel(k_steps<RES_SMALL, true>, grid, tpb, args, smem, s);
-    }
-    if (big) return cudaLaunchCooperativeKernel(k_steps<RES_LARGE, false>, grid, tpb, args, smem, s);
-    return cudaLaunchCooperativeKernel(k_steps<RES_SMALL, false>, grid, tpb, args, smem, s);
+    return cudaLaunchCooperativeKernel(kernel, grid, tpb, args, smem, s);
 }
 void launch_node_cn(cudaStream_t s, const uint32_t* cnode, long long i0, long long i1, uint32_t* node_cn) {
     if (i1 > i0) k_node_cn<<<(unsigned)blocks_for(i1 - i0, TPB), TPB, 0, s>>>(cnode, i0, i1, node_cn);

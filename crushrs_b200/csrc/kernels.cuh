@@ -214,9 +214,9 @@ struct ActiveBuild {
     int* lists;                  // same layout as the chunks
     int* counts;                 // ACTIVE_SPACES
 };
-constexpr int ACTIVE_SPACES = 9;  // honeycomb elements, all elements, nodes, searched entries (dynamic grids and the
+constexpr int ACTIVE_SPACES = 10;  // honeycomb elements, all elements, nodes, searched entries (dynamic grids and the
                                   // rest), contact nodes, moving faces, all primary-node entries, static-grid entries,
-                                  // scalar elements
+                                  // scalar elements, exhaustively searched entries
 
 // Vehicles of all crash slots: node lists and the reduction layout.
 struct VehicleArrays {
@@ -430,7 +430,7 @@ struct ResidentSync {
     int error;            // a block gave up waiting at a barrier
     int pad;
 };
-constexpr int RESIDENT_MAX_SLOTS = 128;  // crashes of one launch (their control views are in shared memory)
+constexpr int RESIDENT_MAX_SLOTS = 1024;  // crashes of one launch (their control views are in shared memory)
 struct ResidentArgs {
     ElementArrays el;     // el_run
     NodeArrays nd[2];     // of even and odd steps (nd_step)
@@ -447,10 +447,13 @@ struct ResidentArgs {
     int n_steps;
     int adaptive, check_steps, any_separation, hist_on;
     long long n_slaves;
+    long long n_busy;     // honeycomb elements of the crashes not known to be done
+    int contact0;         // first contact of those crashes (the ones before it are done)
     int sc_oct;           // elastic elements on eight lanes each (set by the launcher)
     const int* lists;     // active chunk lists (ab.lists), or null: every chunk of every space
     long long space_off[ACTIVE_SPACES];
     long long space_n[ACTIVE_SPACES];
+    int chunk_off[ACTIVE_SPACES + 1];  // the spaces' chunks that hold entities, numbered one after the other
 };
 // Steps [step0, step0 + n_steps) of every slot in one cooperative launch of
 // `blocks` blocks (at most resident_blocks: those that fit the device at once).

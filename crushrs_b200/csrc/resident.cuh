@@ -392,9 +392,11 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
     __shared__ double big_box[6];
     __shared__ int s_state, s_chunks[ACTIVE_SPACES];
     __shared__ uint8_t s_cand[RES_TPB / 32][BRUTE_MAX_FACES + 1];
-    __shared__ ControlView view[RESIDENT_MAX_SLOTS];
-    extern __shared__ double oct_shared[];  // OCT_SHARED per eight threads, when elastic elements take eight lanes
+    // OCT_SHARED per eight threads, when elastic elements take eight lanes, then
+    // a control view per slot
+    extern __shared__ double oct_shared[];
     constexpr int RES_WARPS = RES_TPB / 32;
+    ControlView* view = reinterpret_cast<ControlView*>(oct_shared + (ELASTIC && A.sc_oct ? OCT_SHARED * RES_TPB / 8 : 0));
     static_assert(RES_TPB >= HEAVY_TPB && VEH_TPB == HEAVY_TPB && sizeof(heavy.sf) >= 2 * sizeof(double) * VEH_TPB, "block sums");
     const bool summing = threadIdx.x < HEAVY_TPB;  // the threads of the block-wide sums
     const bool odd_jobs = blockIdx.x == gridDim.x - 1;  // the block that does what one block does
@@ -426,15 +428,29 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
         if (threadIdx.x < ACTIVE_SPACES)
             s_chunks[threadIdx.x] = A.lists ? A.ab.counts[threadIdx.x] : (int)((A.space_n[threadIdx.x] + CHUNK - 1) / CHUNK);
     };
-    auto running = [&] {  // block-wide; orders the view for the block as well
-        int any = 0;
-        for (int sl = threadIdx.x; sl < n_slots; sl += RES_TPB) any |= !view[sl].done;
-        return __syncthreads_or(any) != 0;
+    // The crashes still running, block-wide; orders the view for the block as well.
+    auto running = [&] {
+        int n = 0;
+        for (int sl = 0; sl < n_slots; sl += RES_TPB) n += __syncthreads_count(sl + threadIdx.x < n_slots && !view[sl + threadIdx.x].done);
+        return n;
     };
-    auto rebuild = [&] {  // the chunks that still hold a running crash (one block)
+    // The chunks that still hold a running crash, in one block (over the chunks
+    // that hold entities, not a serving context's whole room: 50,000 chunks of a
+    // room of 2 M elements).
+    auto rebuild = [&] {
         for (int k = threadIdx.x; k < ACTIVE_SPACES; k += RES_TPB) A.ab.counts[k] = 0;
         __syncthreads();
-        for (long long t = threadIdx.x; t - threadIdx.x < A.ab.n_chunks; t += RES_TPB) build_active_body(A.ab, ctls, t);
+        const int total = A.chunk_off[ACTIVE_SPACES];
+        for (int k0 = 0; k0 < total; k0 += RES_TPB) {
+            const int k = k0 + threadIdx.x;
+            long long t = A.ab.n_chunks;  // none
+            if (k < total) {
+                int sp = 0;
+                while (k >= A.chunk_off[sp + 1]) ++sp;
+                t = A.space_off[sp] + (k - A.chunk_off[sp]);
+            }
+            build_active_body(A.ab, ctls, t);
+        }
         __syncthreads();
     };
     auto finalize = [&] {
@@ -473,7 +489,8 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
         if (A.adaptive && A.step0 % A.check_steps == 0) finalize();
     });
     if (go) load_view();
-    go = running() && go;
+    int n_running = running(), n_listed = n_running;  // now, and when the lists were built
+    go = go && n_running > 0;
     TaskDeal deal{(int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x), (int)gridDim.x * RES_WARPS, 0};
     for (int i = 0; go && i < A.n_steps; ++i) {
         const long long step = A.step0 + i;
@@ -575,8 +592,11 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
         deal.base = 0;
 
         // Full update beside the search of the next step's contacts.
-        deal((int)ca.n_brute_entries, [&](int t) {
-            const BruteEntry be = ca.brute_entries[t];
+        deal(tasks(9, 32), [&](int t) {
+            int l;
+            const long long e = entity(9, t, 32, &l);
+            if (e >= ca.n_brute_entries) return;
+            const BruteEntry be = ca.brute_entries[e];
             double sd = 0.0;
             const int best = resident_brute(cn, nd, view, be, lane, s_cand[threadIdx.x >> 5], &sd);
             if (plain) resident_emit<32>(cn, view, nd.mass, be.s, best, sd, lane);
@@ -606,7 +626,8 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             });
         if (grids) {
             if (ca.n_buckets > 0) {
-                deal((int)((ca.n_buckets + 31) / 32), [&](int t) { grid_alloc_body(ca, 0, ca.n_contacts, (long long)t * 32 + lane); });
+                deal((int)((ca.n_buckets - ca.tab_off[A.contact0] + 31) / 32),
+                     [&](int t) { grid_alloc_body(ca, A.contact0, ca.n_contacts, (long long)t * 32 + lane); });
                 contact_big_block(ca, nd, big_face, big_box);
                 if (!(go = barrier(&s_state))) break;
                 deal.base = 0;
@@ -656,16 +677,24 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             }
             pending_end = true;
         } else {
+            // crashes only ever stop during a launch, so the same number is the same lists
+            const bool relist = A.lists && (step + 1) % 20 == 0 && i + 1 < A.n_steps;
             go = barrier(&s_state, [&] {
                 end_step(step, sep);
                 __syncthreads();  // the mass flag is clear before a slot sets it
                 if (check_next && i + 1 < A.n_steps) finalize();
-                if (A.lists && (step + 1) % 20 == 0 && i + 1 < A.n_steps) rebuild();
+                if (relist) {
+                    int n = 0;
+                    for (int sl = 0; sl < n_slots; sl += RES_TPB)
+                        n += __syncthreads_count(sl + threadIdx.x < n_slots && !ctls[sl + threadIdx.x].done);
+                    if (n != n_listed) rebuild();
+                }
             });
             if (!go) break;
             load_view();
         }
-        const bool more = running();
+        n_running = running();
+        if ((step + 1) % 20 == 0) n_listed = n_running;
         if (A.hist_on && (step + 1) % A.hist.steps == 0) {
             deal.base = 0;
             deal(A.hist.n_pu * HIST_BLOCKS, [&](int t) {
@@ -682,7 +711,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             pending_record = true;
             if (!(go = barrier(&s_state))) break;
         }
-        if (!more) break;
+        if (n_running == 0) break;
     }
     if (!go) return;
     // every crash is done, or the launch's last step was not a plain one
