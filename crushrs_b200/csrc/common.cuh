@@ -20,20 +20,8 @@ constexpr int P_CONN = 0;    // 2 planes: node ids 0-3, 4-7 (uint32 bits)
 constexpr int P_GRAD = 2;    // 6 planes: dN/dX at the centre, grad[3 i + c]
 constexpr int P_GAMMA = 8;   // 8 planes: gamma[4 i + a]
 constexpr int P_H = 16;      // 20 planes: upper triangle of H, row-major (78 used)
-constexpr int P_META = 36;   // 1 plane: volume (f32), material index, shape (SHAPE_NONE: none), crash slot
+constexpr int P_META = 36;   // 1 plane: volume (f32), material index, model element index, crash slot
 constexpr int N_STATIC_PLANES = 37;
-// Shape table: the distinct (dN/dX, gamma) records of a context's elements.
-// The blocks that meshes are cut from repeat one box, whose gradients and
-// base vectors are the same 56 floats bit for bit (1 or 2 distinct records
-// on the synthetic head-ons; only H, full of rounding noise around its zeros,
-// differs from element to element), so the element kernel reads them from a
-// few table entries that stay in L1 instead of 224 bytes per element. An
-// element whose record found no entry (a mesh of more shapes than SHAPE_CAP)
-// has SHAPE_NONE and reads its planes.
-constexpr int SHAPE_F4 = P_H - P_GRAD;  // 14 float4 per record, in plane order
-constexpr int SHAPE_CAP = 1024;         // entries (a power of two): 229 KB, what L1 can hold
-constexpr int SHAPE_PROBES = 8;
-constexpr uint32_t SHAPE_NONE = 0xFFFFFFFFu;
 // State: F_prev^-1 (9), R (9), stress (6), compaction, eroded flag (as bits), 2 pad.
 constexpr int N_STATE_PLANES = 7;
 constexpr int S_COMPACTION = 24;

@@ -470,9 +470,6 @@ struct crush_ctx {
     long long* voff_d = nullptr;
     double *sc_geo = nullptr, *sc_mat = nullptr, *sc_corner = nullptr;
     float4 *planes = nullptr, *state = nullptr;
-    float4* shapes = nullptr;                  // shape table of the honeycomb elements and the hashes its entries hold
-    unsigned long long* shape_keys = nullptr;
-    uint32_t* hc_model_d = nullptr;            // per honeycomb element: model element
     float* corner = nullptr;
     MaterialF32* mats = nullptr;
     Control* ctls = nullptr;      // the run, one per slot
@@ -570,8 +567,6 @@ struct crush_ctx {
         e.n_hc = n_hc;
         e.stride = stride;
         e.planes = planes;
-        e.shapes = shapes;
-        e.hc_model = hc_model_d;
         e.state = state;
         e.corner = corner;
         e.mats = mats;
@@ -1633,9 +1628,6 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         TRY(c->alloc(&c->eroded_all, EC));
         TRY(c->alloc(&c->planes, (size_t)N_STATIC_PLANES * c->stride));
         TRY(c->alloc(&c->state, (size_t)N_STATE_PLANES * c->stride));
-        TRY(c->alloc(&c->shapes, (size_t)SHAPE_CAP * SHAPE_F4));
-        TRY(c->alloc(&c->shape_keys, SHAPE_CAP));
-        TRY(c->alloc(&c->hc_model_d, EC));
         TRY(c->alloc(&c->corner, (size_t)24 * EC));
         TRY(c->alloc(&c->sc_geo, (size_t)SC_PLANES * c->sc_stride));
         TRY(c->alloc(&c->sc_corner, (size_t)24 * QC));
@@ -1650,7 +1642,6 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         CK(cudaMemsetAsync(c->fused_counter, 0, sizeof(unsigned), c->stream));
         CK(cudaMemsetAsync(c->forces_queue, 0, 2 * sizeof(unsigned), c->stream));
         CK(cudaMemsetAsync(c->planes, 0, sizeof(float4) * N_STATIC_PLANES * c->stride, c->stream));
-        CK(cudaMemsetAsync(c->shape_keys, 0, sizeof(unsigned long long) * SHAPE_CAP, c->stream));
         CK(cudaMemsetAsync(c->eroded_all, 0, EC, c->stream));
         CK(cudaMemsetAsync(c->ctls, 0, sizeof(Control) * cap.slots, c->stream));
         CK(cudaMemsetAsync(c->slot_done, 0, sizeof(int) * cap.slots, c->stream));
@@ -2000,11 +1991,8 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     trace.mark("node incidence queued");
     CK(cudaMemsetAsync(c->setup_bad, 0, sizeof(int), c->stream));
     launch_setup_geometry(c->stream, E0, E0 + E, c->pos, c->conn_all, c->part, c->mat4, c->hc_index_d, c->elem_slot, c->stride, c->planes,
-                          c->volume, c->lumped, c->dt_factor, c->elem_mass, c->setup_bad, c->sc_index_d, c->sc_stride, c->sc_geo,
-                          c->hc_model_d);
+                          c->volume, c->lumped, c->dt_factor, c->elem_mass, c->setup_bad, c->sc_index_d, c->sc_stride, c->sc_geo);
     TRY(check_launch(c));
-    launch_shapes(c->stream, H0, H0 + H, c->stride, c->planes, c->shape_keys, c->shapes);
-    TRY(check_launch(c, H > 0 ? 2 : 0));
     launch_node_masses(c->stream, N, c->all_off + N0, c->all_slot, c->lumped, c->mass + N0, c->inv_mass + N0);
     TRY(check_launch(c));
     launch_init_state(c->stream, H0, H0 + H, c->stride, c->state);
@@ -2765,7 +2753,6 @@ int begin_slots(crush_ctx* c, int s0, int s1) {
     // the slots' first entries.
     ElementArrays w = c->el();
     w.planes += h0;
-    w.hc_model += h0;
     w.state += h0;
     w.corner += 24 * h0;
     w.n_hc = h1 - h0;

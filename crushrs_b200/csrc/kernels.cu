@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(GEO_TPB) k_setup_geometry8(long long e_begin, 
                                                              double* __restrict__ lumped_out, double* __restrict__ dt_factor,
                                                              double* __restrict__ elem_mass, int* __restrict__ bad,
                                                              const int64_t* __restrict__ sc_index, long long n_sc,
-                                                             double* __restrict__ sc_geo, uint32_t* __restrict__ hc_model) {
+                                                             double* __restrict__ sc_geo) {
     __shared__ double s_gkg[GEO_PER_BLOCK][78];
     __shared__ double s_h[GEO_PER_BLOCK][80];
     const int q = threadIdx.x % GEO_LANES, grp = threadIdx.x / GEO_LANES;
@@ -333,7 +333,6 @@ __global__ void __launch_bounds__(GEO_TPB) k_setup_geometry8(long long e_begin, 
     if (sc >= 0)
         for (int k = q; k < 78; k += GEO_LANES) sc_geo[(SC_H + k) * n_sc + sc] = s_h[grp][k];
     if (h < 0) return;
-    if (q == 0) hc_model[h] = (uint32_t)e;
     // the element's 37 planes, split over the lanes
     for (int k = q; k < N_STATIC_PLANES; k += GEO_LANES) {
         float4 v;
@@ -353,71 +352,10 @@ __global__ void __launch_bounds__(GEO_TPB) k_setup_geometry8(long long e_begin, 
             for (int t = 0; t < 4; ++t) f[t] = o + t < 78 ? (float)s_h[grp][o + t] : 0.0f;
             v = make_float4(f[0], f[1], f[2], f[3]);
         } else {
-            v = make_float4((float)volume, __uint_as_float((uint32_t)p), __uint_as_float(SHAPE_NONE), __uint_as_float(elem_slot[e]));
+            v = make_float4((float)volume, __uint_as_float((uint32_t)p), __uint_as_float((uint32_t)e), __uint_as_float(elem_slot[e]));
         }
         planes[k * stride + h] = v;
     }
-}
-
-// Shape table, claim pass: thread per element, a 64-bit hash of its record
-// looked up with linear probing; the first element of a record claims the
-// entry and writes it. Which entry a record gets may change from run to run,
-// its contents do not.
-__device__ __forceinline__ unsigned long long mix64(unsigned long long h) {
-    h ^= h >> 32;
-    h *= 0xD6E8FEB86659FD93ull;
-    h ^= h >> 32;
-    return h;
-}
-__global__ void k_shape_claim(long long h_begin, long long n_hc, long long stride, float4* __restrict__ planes, unsigned long long* keys,
-                              float4* __restrict__ shapes) {
-    const long long e = h_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_hc) return;
-    uint4 r[SHAPE_F4];
-    unsigned long long h = 0;
-#pragma unroll
-    for (int k = 0; k < SHAPE_F4; ++k) {
-        r[k] = *reinterpret_cast<const uint4*>(planes + (P_GRAD + k) * stride + e);
-        h = mix64(h + (((unsigned long long)r[k].y << 32) | r[k].x));
-        h = mix64(h + (((unsigned long long)r[k].w << 32) | r[k].z));
-    }
-    h |= 1ull;
-    uint32_t sid = SHAPE_NONE;
-    for (int p = 0; p < SHAPE_PROBES; ++p) {
-        const uint32_t slot = ((uint32_t)(h >> 20) + p) & (SHAPE_CAP - 1);
-        unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(keys + slot);
-        if (cur == 0ull) {
-            cur = atomicCAS(keys + slot, 0ull, h);
-            if (cur == 0ull) {
-#pragma unroll
-                for (int k = 0; k < SHAPE_F4; ++k) reinterpret_cast<uint4*>(shapes)[slot * SHAPE_F4 + k] = r[k];
-                cur = h;
-            }
-        }
-        if (cur == h) {
-            sid = slot;
-            break;
-        }
-    }
-    planes[P_META * stride + e].z = __uint_as_float(sid);
-}
-
-// Check pass, after the claims: an element keeps its entry when the record
-// there is its own bit for bit (two records may share a hash).
-__global__ void k_shape_check(long long h_begin, long long n_hc, long long stride, float4* __restrict__ planes,
-                              const float4* __restrict__ shapes) {
-    const long long e = h_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_hc) return;
-    const uint32_t sid = __float_as_uint(planes[P_META * stride + e].z);
-    if (sid == SHAPE_NONE) return;
-    bool same = true;
-#pragma unroll
-    for (int k = 0; k < SHAPE_F4; ++k) {
-        const uint4 a = *reinterpret_cast<const uint4*>(planes + (P_GRAD + k) * stride + e);
-        const uint4 b = *reinterpret_cast<const uint4*>(shapes + sid * SHAPE_F4 + k);
-        same = same && a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
-    }
-    if (!same) planes[P_META * stride + e].z = __uint_as_float(SHAPE_NONE);
 }
 
 // Lumped nodal masses: Σ over incident (element, corner) in element order
@@ -502,15 +440,6 @@ __global__ void k_incidence_split(long long nn, const uint32_t* __restrict__ rel
 
 // ---------------------------------------------------------------------------
 // Element forces (src/kernel_simd.rs:300-491, one element per thread).
-//
-// Bound by the latency and volume of its streams: 2259 instructions per warp
-// fill 47 % of the issue slots, the rest waits for memory at 16 warps per SM.
-// Gradients and Γ come from the shape table (common.cuh; L1) and H streams
-// through four registers, so an element moves 688 B instead of 912 B: one
-// launch on 278,640 elements takes 42.2 us (4.5 TB/s), 52.7 us with the 14
-// planes read and H held in registers. 128 registers and 2 x 256 threads per
-// SM: more warps spill and lose (3 x 256 at 80 registers 53.1 us, 5 x 128 at
-// 96 45.8 us, 6 x 128 at 80 52.4 us).
 // ---------------------------------------------------------------------------
 #ifndef FORCES_TPB
 #define FORCES_TPB 256
@@ -524,59 +453,57 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
     if (e >= el.n_hc) return;
     const long long S = el.stride;
     const float4 meta = ld_plane(el.planes, S, P_META, e);
-    const float4 c0 = ld_plane(el.planes, S, P_CONN, e), c1 = ld_plane(el.planes, S, P_CONN + 1, e);
-    const float4 st6 = el.state[6 * S + e];
     Control* ctl = ctls + __float_as_uint(meta.w);
     if (respect_done && view[__float_as_uint(meta.w)].done) return;
     float4* out = reinterpret_cast<float4*>(el.corner + 24 * e);
+    const float4 st6 = el.state[6 * S + e];
     if (__float_as_uint(st6.y) != 0u) {  // already eroded: no force
         for (int k = 0; k < 6; ++k) out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
+    const float4 c0 = ld_plane(el.planes, S, P_CONN, e), c1 = ld_plane(el.planes, S, P_CONN + 1, e);
     const uint32_t nid[8] = {__float_as_uint(c0.x), __float_as_uint(c0.y), __float_as_uint(c0.z), __float_as_uint(c0.w),
                              __float_as_uint(c1.x), __float_as_uint(c1.y), __float_as_uint(c1.z), __float_as_uint(c1.w)};
-    // dN/dX and Γ from the shape table, or the element's own planes
-    const uint32_t sid = __float_as_uint(meta.z);
-    const float4* shape = sid != SHAPE_NONE ? el.shapes + sid * SHAPE_F4 : el.planes + P_GRAD * S + e;
-    const long long sstep = sid != SHAPE_NONE ? 1 : S;
+    float grad[24];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        float4 g = ld_plane(el.planes, S, P_GRAD + k, e);
+        grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
+    }
+    float gam[32];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float4 g = ld_plane(el.planes, S, P_GAMMA + k, e);
+        gam[4 * k] = g.x; gam[4 * k + 1] = g.y; gam[4 * k + 2] = g.z; gam[4 * k + 3] = g.w;
+    }
     // F = Σ x_i ⊗ ∇N_i with x = (X + u) as f32; q = U Γ with u as f32.
     M3f f;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) f.m[k] = 0.0f;
     float q[12];
-    {
-        float grad[24];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            const float4 g = __ldg(shape + k * sstep);
-            grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
-        }
+    for (int k = 0; k < 12; ++k) q[k] = 0.0f;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) f.m[k] = 0.0f;
+    for (int i = 0; i < 8; ++i) {
+        const long long n = nid[i];
+        const double* P = nd.pos + 3 * n;
+        const double* U = nd.u + 3 * n;
+        const double u0 = U[0], u1 = U[1], u2 = U[2];
+        const float x[3] = {(float)(__ldg(P) + u0), (float)(__ldg(P + 1) + u1), (float)(__ldg(P + 2) + u2)};
+        const float ul[3] = {(float)u0, (float)u1, (float)u2};
 #pragma unroll
-        for (int k = 0; k < 12; ++k) q[k] = 0.0f;
+        for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const long long n = nid[i];
-            const double* P = nd.pos + 3 * n;
-            const double* U = nd.u + 3 * n;
-            const double u0 = U[0], u1 = U[1], u2 = U[2];
-            const float x[3] = {(float)(__ldg(P) + u0), (float)(__ldg(P + 1) + u1), (float)(__ldg(P + 2) + u2)};
-            const float ul[3] = {(float)u0, (float)u1, (float)u2};
+            for (int c = 0; c < 3; ++c) f.m[3 * a + c] = x[a] * grad[3 * i + c] + f.m[3 * a + c];
 #pragma unroll
-            for (int a = 0; a < 3; ++a)
+        for (int mode = 0; mode < 4; ++mode)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) f.m[3 * a + c] = x[a] * grad[3 * i + c] + f.m[3 * a + c];
-            const float4 g4 = __ldg(shape + (6 + i) * sstep);
-            const float gam[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-            for (int mode = 0; mode < 4; ++mode)
-#pragma unroll
-                for (int dir = 0; dir < 3; ++dir) q[3 * mode + dir] = ul[dir] * gam[mode] + q[3 * mode + dir];
-        }
+            for (int dir = 0; dir < 3; ++dir) q[3 * mode + dir] = ul[dir] * gam[4 * i + mode] + q[3 * mode + dir];
     }
     const float det = det3(f);
     if (det <= 0.0f) {  // inverted: erode (src/kernel_simd.rs:324-331)
         el.state[6 * S + e] = make_float4(st6.x, __uint_as_float(1u), st6.z, st6.w);
-        el.eroded_all[el.hc_model[e]] = 1;
+        el.eroded_all[__float_as_uint(meta.z)] = 1;
         atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->eroded_step), 1ull);
         for (int k = 0; k < 6; ++k) out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
@@ -599,50 +526,39 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
     const float vol = meta.x;
 #pragma unroll
     for (int k = 0; k < 9; ++k) m.m[k] = m.m[k] * vol;
-    // Hourglass: rr = H q, every row's sum in column order. The upper
-    // triangle streams by in row order: entry (i, j) is column j of row i and
-    // column i of row j, and a row's columns below its own come from the
-    // rows before it, so one pass keeps the order with four entries live.
-    float rr[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) rr[k] = 0.0f;
-    {
-        float h4[4];
-        int idx = 0;
-#pragma unroll
-        for (int i = 0; i < 12; ++i)
-#pragma unroll
-            for (int j = i; j < 12; ++j, ++idx) {
-                if (idx % 4 == 0) {
-                    const float4 h = ld_plane(el.planes, S, P_H + idx / 4, e);
-                    h4[0] = h.x; h4[1] = h.y; h4[2] = h.z; h4[3] = h.w;
-                }
-                rr[i] = h4[idx % 4] * q[j] + rr[i];
-                if (j > i) rr[j] = h4[idx % 4] * q[i] + rr[j];
-            }
-    }
-    // f_i += rr Γᵀ, gradients and Γ read again (L1) instead of kept in registers
-    float grad[24];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const float4 g = __ldg(shape + k * sstep);
-        grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
-    }
     float fo[24];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float4 g4 = __ldg(shape + (6 + i) * sstep);
-        const float gam[4] = {g4.x, g4.y, g4.z, g4.w};
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             float acc = m.m[3 * a] * grad[3 * i];
             acc = m.m[3 * a + 1] * grad[3 * i + 1] + acc;
             acc = m.m[3 * a + 2] * grad[3 * i + 2] + acc;
-#pragma unroll
-            for (int mode = 0; mode < 4; ++mode) acc = rr[3 * mode + a] * gam[mode] + acc;
             fo[3 * i + a] = acc;
         }
+    // Hourglass: rr = H q (column order), f += rr Γᵀ.
+    float hsym[80];
+#pragma unroll
+    for (int k = 0; k < 20; ++k) {
+        float4 h4 = ld_plane(el.planes, S, P_H + k, e);
+        hsym[4 * k] = h4.x; hsym[4 * k + 1] = h4.y; hsym[4 * k + 2] = h4.z; hsym[4 * k + 3] = h4.w;
     }
+    float rr[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) rr[k] = 0.0f;
+#pragma unroll
+    for (int col = 0; col < 12; ++col)
+#pragma unroll
+        for (int row = 0; row < 12; ++row) rr[row] = hsym[h_index(row, col)] * q[col] + rr[row];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int dir = 0; dir < 3; ++dir) {
+            float acc = fo[3 * i + dir];
+#pragma unroll
+            for (int mode = 0; mode < 4; ++mode) acc = rr[3 * mode + dir] * gam[4 * i + mode] + acc;
+            fo[3 * i + dir] = acc;
+        }
 #pragma unroll
     for (int k = 0; k < 6; ++k) out[k] = make_float4(fo[4 * k], fo[4 * k + 1], fo[4 * k + 2], fo[4 * k + 3]);
 }
@@ -2441,18 +2357,11 @@ void launch_node_cn(cudaStream_t s, const uint32_t* cnode, long long i0, long lo
 void launch_setup_geometry(cudaStream_t s, long long e_begin, long long n_all, const double* pos, const uint32_t* conn_all,
                            const int32_t* part, const double* mat, const int64_t* hc_index, const uint32_t* elem_slot, long long stride,
                            float4* planes, double* volume, double* lumped, double* dt_factor, double* elem_mass, int* bad,
-                           const int64_t* sc_index, long long n_sc, double* sc_geo, uint32_t* hc_model) {
+                           const int64_t* sc_index, long long n_sc, double* sc_geo) {
     if (n_all <= e_begin) return;
     k_setup_geometry8<<<(unsigned)blocks_for(n_all - e_begin, GEO_PER_BLOCK), GEO_TPB, 0, s>>>(
         e_begin, n_all, pos, conn_all, part, mat, hc_index, elem_slot, stride, planes, volume, lumped, dt_factor, elem_mass, bad, sc_index,
-        n_sc, sc_geo, hc_model);
-}
-void launch_shapes(cudaStream_t s, long long h_begin, long long n_hc, long long stride, float4* planes, unsigned long long* keys,
-                   float4* shapes) {
-    if (n_hc <= h_begin) return;
-    const unsigned g = (unsigned)blocks_for(n_hc - h_begin, TPB);
-    k_shape_claim<<<g, TPB, 0, s>>>(h_begin, n_hc, stride, planes, keys, shapes);
-    k_shape_check<<<g, TPB, 0, s>>>(h_begin, n_hc, stride, planes, shapes);
+        n_sc, sc_geo);
 }
 void launch_node_masses(cudaStream_t s, long long n, const uint32_t* off, const uint32_t* slot, const double* lumped,
                         double* mass, double* inv_mass) {

@@ -20,8 +20,6 @@ struct ElementArrays {
     long long n_hc;          // honeycomb elements
     long long stride;        // plane stride (n_hc rounded up)
     const float4* planes;    // N_STATIC_PLANES * stride
-    const float4* shapes;    // SHAPE_CAP * SHAPE_F4: the shape table (common.cuh)
-    const uint32_t* hc_model;  // per honeycomb element: model element
     float4* state;           // N_STATE_PLANES * stride
     float* corner;           // 24 floats per honeycomb element (corner forces)
     const MaterialF32* mats;
@@ -235,12 +233,7 @@ void launch_setup_geometry(cudaStream_t s, long long e_begin, long long n_all, c
                            const int32_t* part, const double* mat_e_nu_rho_hg, const int64_t* hc_index,
                            const uint32_t* elem_slot, long long stride, float4* planes, double* volume, double* lumped,
                            double* dt_factor, double* elem_mass, int* bad, const int64_t* sc_index, long long n_sc,
-                           double* sc_geo, uint32_t* hc_model);
-// Shape table entries of honeycomb elements [h_begin, n_hc): every element's
-// record finds or claims an entry of `shapes` (keys: SHAPE_CAP hashes, 0 =
-// free) and its meta plane gets the entry's index. Two launches.
-void launch_shapes(cudaStream_t s, long long h_begin, long long n_hc, long long stride, float4* planes, unsigned long long* keys,
-                   float4* shapes);
+                           double* sc_geo);
 void launch_node_masses(cudaStream_t s, long long n, const uint32_t* off, const uint32_t* slot, const double* lumped,
                         double* mass, double* inv_mass);
 void launch_init_state(cudaStream_t s, long long h_begin, long long n_hc, long long stride, float4* state);
