@@ -440,6 +440,13 @@ __global__ void k_incidence_split(long long nn, const uint32_t* __restrict__ rel
 
 // ---------------------------------------------------------------------------
 // Element forces (src/kernel_simd.rs:300-491, one element per thread).
+//
+// Bound by memory latency at 16 warps per SM (128 registers, 2 x 256 threads).
+// H streams through four registers instead of being held in 80, and gradients
+// and Γ are loaded where they are used, twice: the second read of these 224 B
+// comes from L1 (112 KB per SM in flight). A device force call on 278,640
+// elements takes 65.1 us, 67.9 us with everything held; held gradients and Γ
+// with H streamed 67.6 us.
 // ---------------------------------------------------------------------------
 #ifndef FORCES_TPB
 #define FORCES_TPB 256
@@ -453,52 +460,51 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
     if (e >= el.n_hc) return;
     const long long S = el.stride;
     const float4 meta = ld_plane(el.planes, S, P_META, e);
+    const float4 c0 = ld_plane(el.planes, S, P_CONN, e), c1 = ld_plane(el.planes, S, P_CONN + 1, e);
+    const float4 st6 = el.state[6 * S + e];
     Control* ctl = ctls + __float_as_uint(meta.w);
     if (respect_done && view[__float_as_uint(meta.w)].done) return;
     float4* out = reinterpret_cast<float4*>(el.corner + 24 * e);
-    const float4 st6 = el.state[6 * S + e];
     if (__float_as_uint(st6.y) != 0u) {  // already eroded: no force
         for (int k = 0; k < 6; ++k) out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    const float4 c0 = ld_plane(el.planes, S, P_CONN, e), c1 = ld_plane(el.planes, S, P_CONN + 1, e);
     const uint32_t nid[8] = {__float_as_uint(c0.x), __float_as_uint(c0.y), __float_as_uint(c0.z), __float_as_uint(c0.w),
                              __float_as_uint(c1.x), __float_as_uint(c1.y), __float_as_uint(c1.z), __float_as_uint(c1.w)};
-    float grad[24];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        float4 g = ld_plane(el.planes, S, P_GRAD + k, e);
-        grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
-    }
-    float gam[32];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        float4 g = ld_plane(el.planes, S, P_GAMMA + k, e);
-        gam[4 * k] = g.x; gam[4 * k + 1] = g.y; gam[4 * k + 2] = g.z; gam[4 * k + 3] = g.w;
-    }
+    const float4* geo = el.planes + P_GRAD * S + e;  // dN/dX and Γ
     // F = Σ x_i ⊗ ∇N_i with x = (X + u) as f32; q = U Γ with u as f32.
     M3f f;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) f.m[k] = 0.0f;
     float q[12];
+    {
+        float grad[24];
 #pragma unroll
-    for (int k = 0; k < 12; ++k) q[k] = 0.0f;
+        for (int k = 0; k < 6; ++k) {
+            const float4 g = __ldg(geo + k * S);
+            grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
+        }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const long long n = nid[i];
-        const double* P = nd.pos + 3 * n;
-        const double* U = nd.u + 3 * n;
-        const double u0 = U[0], u1 = U[1], u2 = U[2];
-        const float x[3] = {(float)(__ldg(P) + u0), (float)(__ldg(P + 1) + u1), (float)(__ldg(P + 2) + u2)};
-        const float ul[3] = {(float)u0, (float)u1, (float)u2};
+        for (int k = 0; k < 9; ++k) f.m[k] = 0.0f;
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < 12; ++k) q[k] = 0.0f;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) f.m[3 * a + c] = x[a] * grad[3 * i + c] + f.m[3 * a + c];
+        for (int i = 0; i < 8; ++i) {
+            const long long n = nid[i];
+            const double* P = nd.pos + 3 * n;
+            const double* U = nd.u + 3 * n;
+            const double u0 = U[0], u1 = U[1], u2 = U[2];
+            const float x[3] = {(float)(__ldg(P) + u0), (float)(__ldg(P + 1) + u1), (float)(__ldg(P + 2) + u2)};
+            const float ul[3] = {(float)u0, (float)u1, (float)u2};
 #pragma unroll
-        for (int mode = 0; mode < 4; ++mode)
+            for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int dir = 0; dir < 3; ++dir) q[3 * mode + dir] = ul[dir] * gam[4 * i + mode] + q[3 * mode + dir];
+                for (int c = 0; c < 3; ++c) f.m[3 * a + c] = x[a] * grad[3 * i + c] + f.m[3 * a + c];
+            const float4 g4 = __ldg(geo + (6 + i) * S);
+            const float gam[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+            for (int mode = 0; mode < 4; ++mode)
+#pragma unroll
+                for (int dir = 0; dir < 3; ++dir) q[3 * mode + dir] = ul[dir] * gam[mode] + q[3 * mode + dir];
+        }
     }
     const float det = det3(f);
     if (det <= 0.0f) {  // inverted: erode (src/kernel_simd.rs:324-331)
@@ -526,39 +532,50 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
     const float vol = meta.x;
 #pragma unroll
     for (int k = 0; k < 9; ++k) m.m[k] = m.m[k] * vol;
+    // Hourglass: rr = H q, every row's sum in column order. The upper
+    // triangle streams by in row order: entry (i, j) is column j of row i and
+    // column i of row j, and a row's columns below its own come from the
+    // rows before it, so one pass keeps the order with four entries live.
+    float rr[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) rr[k] = 0.0f;
+    {
+        float h4[4];
+        int idx = 0;
+#pragma unroll
+        for (int i = 0; i < 12; ++i)
+#pragma unroll
+            for (int j = i; j < 12; ++j, ++idx) {
+                if (idx % 4 == 0) {
+                    const float4 h = ld_plane(el.planes, S, P_H + idx / 4, e);
+                    h4[0] = h.x; h4[1] = h.y; h4[2] = h.z; h4[3] = h.w;
+                }
+                rr[i] = h4[idx % 4] * q[j] + rr[i];
+                if (j > i) rr[j] = h4[idx % 4] * q[i] + rr[j];
+            }
+    }
+    // f_i += rr Γᵀ, gradients and Γ read again (L1) instead of kept in registers
+    float grad[24];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const float4 g = __ldg(geo + k * S);
+        grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
+    }
     float fo[24];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < 8; ++i) {
+        const float4 g4 = __ldg(geo + (6 + i) * S);
+        const float gam[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             float acc = m.m[3 * a] * grad[3 * i];
             acc = m.m[3 * a + 1] * grad[3 * i + 1] + acc;
             acc = m.m[3 * a + 2] * grad[3 * i + 2] + acc;
+#pragma unroll
+            for (int mode = 0; mode < 4; ++mode) acc = rr[3 * mode + a] * gam[mode] + acc;
             fo[3 * i + a] = acc;
         }
-    // Hourglass: rr = H q (column order), f += rr Γᵀ.
-    float hsym[80];
-#pragma unroll
-    for (int k = 0; k < 20; ++k) {
-        float4 h4 = ld_plane(el.planes, S, P_H + k, e);
-        hsym[4 * k] = h4.x; hsym[4 * k + 1] = h4.y; hsym[4 * k + 2] = h4.z; hsym[4 * k + 3] = h4.w;
     }
-    float rr[12];
-#pragma unroll
-    for (int k = 0; k < 12; ++k) rr[k] = 0.0f;
-#pragma unroll
-    for (int col = 0; col < 12; ++col)
-#pragma unroll
-        for (int row = 0; row < 12; ++row) rr[row] = hsym[h_index(row, col)] * q[col] + rr[row];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int dir = 0; dir < 3; ++dir) {
-            float acc = fo[3 * i + dir];
-#pragma unroll
-            for (int mode = 0; mode < 4; ++mode) acc = rr[3 * mode + dir] * gam[4 * i + mode] + acc;
-            fo[3 * i + dir] = acc;
-        }
 #pragma unroll
     for (int k = 0; k < 6; ++k) out[k] = make_float4(fo[4 * k], fo[4 * k + 1], fo[4 * k + 2], fo[4 * k + 3]);
 }
@@ -881,7 +898,7 @@ __global__ void __launch_bounds__(SC_TPB) k_forces_scalar(ElementArrays el, Node
 // honeycomb elements each, the rest 8 elastic ones on eight lanes each. Small
 // blocks spread a few elements over the SMs, and the elastic elements (a
 // road's 360 took a launch of their own behind the others) run beside them: a
-// force call on 1290 + 264 elements takes 7.4 us, 12.3 us in three launches.
+// force call on 1290 + 264 elements takes 6.1 us, 12.3 us in three launches.
 constexpr int SMALL_TPB = 64;
 __global__ void __launch_bounds__(SMALL_TPB) k_forces_small(ElementArrays el, NodeArrays nd, Control* ctls, int respect_done, int hc_blocks) {
     __shared__ double sh[SMALL_TPB / 8][OCT_SHARED];
