@@ -441,7 +441,8 @@ __global__ void k_incidence_split(long long nn, const uint32_t* __restrict__ rel
 // ---------------------------------------------------------------------------
 // Element forces (src/kernel_simd.rs:300-491, one element per thread).
 //
-// Bound by memory latency at 16 warps per SM (128 registers, 2 x 256 threads).
+// Bound by memory latency at 16 warps per SM (128 registers, 2 x 256 threads;
+// the figures are of that persistent wave).
 // H streams through four registers instead of being held in 80, and gradients
 // and Γ are loaded where they are used, twice: the second read of these 224 B
 // comes from L1 (112 KB per SM in flight). A device force call on 278,640
@@ -894,7 +895,7 @@ __global__ void __launch_bounds__(SC_TPB) k_forces_scalar(ElementArrays el, Node
     }
 }
 
-// Both kinds of a small mesh in one launch: blocks [0, hc_blocks) take 64
+// Both kinds of a mesh in one launch: blocks [0, hc_blocks) take 64
 // honeycomb elements each, the rest 8 elastic ones on eight lanes each. Small
 // blocks spread a few elements over the SMs, and the elastic elements (a
 // road's 360 took a launch of their own behind the others) run beside them: a
