@@ -405,6 +405,11 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
     Control* ctls = A.ctls;
     const int n_slots = A.ca[0].n_slots;
     const bool contacts = A.ca[0].n_contacts > 0, grids = A.ca[0].n_grid_slaves > 0;
+    // The dynamic grids' three passes (count with the geometry, allocate,
+    // insert) run all or none: a count that no insert takes back would add to
+    // the next search's. None without an entry to look up (bodies that miss
+    // each other, or start apart by more than the contact's reach).
+    const bool cells = grids && A.ca[0].n_buckets > 0;
     ResidentBarrier barrier{A.sync, 0, 0};
     // emitted: the search emitted this step's events. pending_end: the last
     // step's end is still to be written to the control blocks. pending_record:
@@ -576,7 +581,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                 const long long k = entity(8, t, 1, &l);
                 scalar_force_body<true>(el, nd, ctls, view, 1, k < el.n_sc ? (long long)el.sc_list[k] : el.sc_count);
             });
-        if (ca.n_buckets > 0)
+        if (cells)
             deal(tasks(5, FACE_LANES), [&](int t) {
                 int l;
                 const long long k = entity(5, t, FACE_LANES, &l);
@@ -625,7 +630,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                 nonfinite_body(nd, ctls, view, entity(2, t, 1, &l));
             });
         if (grids) {
-            if (ca.n_buckets > 0) {
+            if (cells) {
                 deal((int)((ca.n_buckets - ca.tab_off[A.contact0] + 31) / 32),
                      [&](int t) { grid_alloc_body(ca, A.contact0, ca.n_contacts, (long long)t * 32 + lane); });
                 contact_big_block(ca, nd, big_face, big_box);
