@@ -476,6 +476,7 @@ struct crush_ctx {
     Control* ctls_aux = nullptr;  // drop-in calls, one per slot
     int* slot_done = nullptr;     // per slot: done flag mirrored by the step-end kernel
     ActiveBuild ab{};             // active chunk lists of the run
+    bool lists_built = false;     // they hold every running slot's chunks (a lone crash's resident steps need none)
     std::vector<long long> space_off_h;
     std::vector<int> done_h;
 
@@ -2059,6 +2060,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
     }
     drop_graphs(c);
     if (!c->run_open) return CRUSH_OK;
+    c->lists_built = false;
     TRY(begin_slots(c, S0, c->n_slots));
     // The main stream: the set-up done, the chunk tables, then the new
     // contacts' first search (its scratch is shared with the steps').
@@ -2637,6 +2639,7 @@ int run_begin(crush_ctx* c) {
     c->prologue_done = false;
     c->contact_done = false;
     c->res_used = false;
+    c->lists_built = false;
     if (c->n_contacts > 0) {
         CK(cudaMemsetAsync(c->ca.big_best, 0x7F, sizeof(int) * std::max<long long>(c->n_slaves, 1), c->stream));  // BIG_NONE
         CK(cudaMemsetAsync(c->ca.pen_count, 0, sizeof(unsigned long long) * 2 * c->pen_stride, c->stream));
@@ -2924,7 +2927,25 @@ bool resident(const crush_ctx* c) {
            busy_elements(c, nullptr) + c->n_sc_free <= RESIDENT_MAX_ELEMENTS && c->n_slots <= RESIDENT_MAX_SLOTS;
 }
 
+// The active chunk lists before steps that read them: a step at a multiple of
+// 20 builds them itself, any other needs those of a step before it — which
+// there are none of when the steps so far were a lone crash's resident ones,
+// or slots joined in between.
+int lists_for_steps(crush_ctx* c) {
+    if (!c->lists_built && c->host_step % 20 != 0) {
+        launch_build_active(c->stream, c->ab, c->ctls);
+        const int st = check_launch(c);
+        if (st != CRUSH_OK) return st;
+    }
+    c->lists_built = true;
+    return CRUSH_OK;
+}
+
 int resident_steps(crush_ctx* c, long long n) {
+    if (c->n_slots > 1) {
+        const int st = lists_for_steps(c);
+        if (st != CRUSH_OK) return st;
+    }
     ResidentArgs a;
     a.el = c->el_run();
     for (int k = 0; k < 2; ++k) {
@@ -2987,6 +3008,8 @@ int issue_steps(crush_ctx* c, long long n_steps) {
             if (st != CRUSH_OK) return st;
             c->last_tune_step = c->host_step;
         }
+        st = lists_for_steps(c);
+        if (st != CRUSH_OK) return st;
         // A graph that is not built yet is built for an issue of two periods
         // or more, or at the second period since the graphs were dropped:
         // the first single period after slots joined is launched step by
