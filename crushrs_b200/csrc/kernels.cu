@@ -2328,6 +2328,16 @@ __global__ void k_node_cn(const uint32_t* __restrict__ cnode, long long i0, long
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
+// Dynamic shared memory of a launch with `slots` control views, its elastic
+// elements on eight lanes each or not, and the most that any launch takes.
+size_t resident_smem(int slots, int tpb, bool oct) { return sizeof(ControlView) * (size_t)slots + (oct ? sizeof(double) * OCT_SHARED / 8 * tpb : 0); }
+// A kernel's limit belongs to the device, not to a context: it is only ever
+// set to the most, so that threads that launch with different slot counts do
+// not take it away from one another. (Set anew for a launch past the default:
+// a device reset between two contexts drops it.)
+cudaError_t allow_resident_smem(const void* kernel, int tpb, bool elastic) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)resident_smem(RESIDENT_MAX_SLOTS, tpb, elastic));
+}
 // Asked once per device (the queries take some 0.2 ms).
 int resident_blocks(int device, int n_sms) {
     constexpr int DEVICES = 64;
@@ -2336,14 +2346,14 @@ int resident_blocks(int device, int n_sms) {
     const auto ask = [&] {
         int coop = 0, per_sm = 0;
         if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) return false;
-        const auto fits = [&](auto kernel, int tpb, size_t bytes) {
-            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess &&
-                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tpb, bytes) == cudaSuccess && per_sm >= 1;
+        const auto fits = [&](const void* kernel, int tpb, bool elastic) {
+            return allow_resident_smem(kernel, tpb, elastic) == cudaSuccess &&
+                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tpb, resident_smem(RESIDENT_MAX_SLOTS, tpb, elastic)) ==
+                       cudaSuccess &&
+                   per_sm >= 1;
         };
-        const size_t oct = sizeof(double) * OCT_SHARED / 8, views = sizeof(ControlView) * RESIDENT_MAX_SLOTS;  // oct: per thread
-        return fits(k_steps<RES_SMALL, false>, RES_SMALL, views) && fits(k_steps<RES_LARGE, false>, RES_LARGE, views) &&
-               fits(k_steps<RES_SMALL, true>, RES_SMALL, views + oct * RES_SMALL) &&
-               fits(k_steps<RES_LARGE, true>, RES_LARGE, views + oct * RES_LARGE);
+        return fits((const void*)k_steps<RES_SMALL, false>, RES_SMALL, false) && fits((const void*)k_steps<RES_LARGE, false>, RES_LARGE, false) &&
+               fits((const void*)k_steps<RES_SMALL, true>, RES_SMALL, true) && fits((const void*)k_steps<RES_LARGE, true>, RES_LARGE, true);
     };
     const bool yes = ask();
     if (device >= 0 && device < DEVICES) known[device].store(yes ? 2 : 1);
@@ -2358,13 +2368,13 @@ cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks) {
     b.sc_oct = a.el.n_sc > 0 && wide <= large ? 1 : 0;
     const bool big = b.sc_oct ? wide > small : a.n_busy > small;
     void* args[] = {&b};
-    const size_t smem = (b.sc_oct ? sizeof(double) * OCT_SHARED * (big ? RES_LARGE : RES_SMALL) / 8 : 0) +
-                        sizeof(ControlView) * (size_t)a.ca[0].n_slots;
-    const dim3 grid((unsigned)blocks), tpb(big ? RES_LARGE : RES_SMALL);
+    const int threads = big ? RES_LARGE : RES_SMALL;
+    const size_t smem = resident_smem(a.ca[0].n_slots, threads, b.sc_oct);
+    const dim3 grid((unsigned)blocks), tpb((unsigned)threads);
     const void* kernel = a.el.n_sc > 0 ? (big ? (const void*)k_steps<RES_LARGE, true> : (const void*)k_steps<RES_SMALL, true>)
                                        : (big ? (const void*)k_steps<RES_LARGE, false> : (const void*)k_steps<RES_SMALL, false>);
-    if (smem > 12 * 1024) {  // past the default beside the static part; set anew each time: a device reset between two contexts drops it
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 12 * 1024) {  // past the default beside the static part
+        const cudaError_t e = allow_resident_smem(kernel, threads, a.el.n_sc > 0);
         if (e != cudaSuccess) return e;
     }
     return cudaLaunchCooperativeKernel(kernel, grid, tpb, args, smem, s);
