@@ -538,7 +538,8 @@ struct crush_ctx {
     bool fused_contact_side = false;      // a fused step's next contact forces on the side stream (else main, after the forces)
     ResidentSync* res_sync = nullptr;     // device: the resident step kernel's barrier and outcome
     int res_blocks = 0;                   // blocks of it the device holds at once (0: none)
-    bool res_used = false;                // it ran since the run began
+    bool res_unread = false;              // it was launched since its outcome was last read
+    int res_polls = RESIDENT_POLLS;       // of its barriers before a block gives up
     unsigned* forces_queue = nullptr;     // device: chunk queue of the persistent element-kernel waves
     // Slots added to an open run are set up on `setup`, beside the steps
     // issued last (the set-up writes only the new slots' ranges); the main
@@ -2638,7 +2639,8 @@ int run_begin(crush_ctx* c) {
     CK(cudaMemsetAsync(c->fused_counter, 0, sizeof(unsigned), c->stream));
     c->prologue_done = false;
     c->contact_done = false;
-    c->res_used = false;
+    c->res_unread = false;
+    CK(cudaMemsetAsync(c->res_sync, 0, sizeof(ResidentSync), c->stream));
     c->lists_built = false;
     if (c->n_contacts > 0) {
         CK(cudaMemsetAsync(c->ca.big_best, 0x7F, sizeof(int) * std::max<long long>(c->n_slaves, 1), c->stream));  // BIG_NONE
@@ -2980,12 +2982,13 @@ int resident_steps(crush_ctx* c, long long n) {
         a.space_n[k] = ns[k];
         a.chunk_off[k + 1] = a.chunk_off[k] + (int)((ns[k] + CHUNK - 1) / CHUNK);
     }
-    CK(cudaMemsetAsync(c->res_sync, 0, sizeof(ResidentSync), c->stream));
+    a.polls = c->res_polls;
+    CK(cudaMemsetAsync(c->res_sync, 0, offsetof(ResidentSync, error), c->stream));
     CK(launch_resident(c->stream, a, c->res_blocks));
-    c->res_used = true;
+    c->res_unread = true;
     c->host_step += n;
     c->last_was_graph = false;
-    return check_launch(c);
+    return check_launch(c, RESIDENT_LAUNCHES);
 }
 
 // Issue n_steps steps (graphs where the step index is on a period boundary).
@@ -3046,14 +3049,26 @@ int issue_steps(crush_ctx* c, long long n_steps) {
     return CRUSH_OK;
 }
 
+// Whether the resident steps issued so far went through (synchronises when
+// some were issued since the last look): a run that gave up has no state or
+// results to read, until it begins anew.
+int resident_outcome(crush_ctx* c) {
+    if (!c->res_unread) return CRUSH_OK;
+    int error = 0;
+    CK(cudaMemcpyAsync(&error, &c->res_sync->error, sizeof(error), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    if (error) return crush::fail(CRUSH_ERR_TIMEOUT, "a block of the resident step kernel gave up waiting at its barrier");
+    c->res_unread = false;
+    return CRUSH_OK;
+}
+
 // Whether every slot has finished (device flags read back; synchronises).
 int all_done(crush_ctx* c, int* done) {
     c->done_h.resize(c->n_slots);
     CK(cudaMemcpyAsync(c->done_h.data(), c->slot_done, sizeof(int) * c->n_slots, cudaMemcpyDeviceToHost, c->stream));
-    ResidentSync rs{};
-    if (c->res_used) CK(cudaMemcpyAsync(&rs, c->res_sync, sizeof(rs), cudaMemcpyDeviceToHost, c->stream));
+    const int st = resident_outcome(c);
+    if (st != CRUSH_OK) return st;
     CK(cudaStreamSynchronize(c->stream));
-    if (rs.error) return crush::fail(CRUSH_ERR_TIMEOUT, "a block of the resident step kernel gave up waiting at its barrier");
     int d = 1;
     for (int x : c->done_h) d &= x ? 1 : 0;
     *done = d;
@@ -3075,6 +3090,8 @@ int run_steps(crush_ctx* c, long long n_steps, int* done) {
 // per-vehicle arithmetic on the host (src/bin/crushrs.rs:237-271).
 int results_range(crush_ctx* c, int s0, int s1, crush_results* r) {
     if (s0 < 0 || s1 > c->n_slots || s0 >= s1) return crush::fail(CRUSH_ERR_INVALID, "slot out of range");
+    int st = resident_outcome(c);
+    if (st != CRUSH_OK) return st;
     std::vector<Control> h(s1 - s0);
     CK(cudaMemcpyAsync(h.data(), c->ctls + s0, sizeof(Control) * h.size(), cudaMemcpyDeviceToHost, c->stream));
     // only the vehicles of slots [s0, s1) (consecutive, in slot order) and their crush-measure nodes
@@ -3089,7 +3106,7 @@ int results_range(crush_ctx* c, int s0, int s1, crush_results* r) {
         vr.local += v0;
         launch_vehicle_sums(c->stream, vr, c->mass, c->v, c->v0, c->veh_out + 7 * (size_t)v0);
         launch_gather_ux(c->stream, (long long)(q1 - q0), c->crush_nodes + q0, c->u, c->crush_ux + q0);
-        int st = check_launch(c, 2);
+        st = check_launch(c, 2);
         if (st != CRUSH_OK) return st;
         CK(cudaMemcpyAsync(sums.data() + 7 * (size_t)v0, c->veh_out + 7 * (size_t)v0, sizeof(double) * 7 * (v1 - v0), cudaMemcpyDeviceToHost,
                            c->stream));
@@ -3503,9 +3520,11 @@ int crush_element_data(crush_ctx* c, float* grad, float* volume, float* gamma, f
 
 int crush_get_state(crush_ctx* c, float* state, uint8_t* eroded) {
     if (!c) return crush::fail(CRUSH_ERR_INVALID, "null context");
+    int st = resident_outcome(c);
+    if (st != CRUSH_OK) return st;
     std::vector<float4> sp((size_t)N_STATE_PLANES * c->stride);
     CK(cudaMemcpyAsync(sp.data(), c->state, sizeof(float4) * sp.size(), cudaMemcpyDeviceToHost, c->stream));
-    int st = sync(c);
+    st = sync(c);
     if (st != CRUSH_OK) return st;
     for (long long e = 0; e < c->n_hc; ++e)
         for (int k = 0; k < 26; ++k) {
@@ -3643,7 +3662,8 @@ int crush_history_counts(crush_ctx* c, int slot, int64_t* n_records, int* n_part
     const bool on = c->hist_on && c->hist_ran && slot < (int)c->hist_steps.size() && c->hist_steps[slot] > 0;
     long long count = 0;
     if (on) {
-        int st = history_final(c);
+        int st = resident_outcome(c);
+        if (st == CRUSH_OK) st = history_final(c);
         if (st != CRUSH_OK) return st;
         CK(cudaMemcpyAsync(&count, c->hist.rec_count + slot, sizeof(count), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -3838,6 +3858,12 @@ int crush_set_contact_search(crush_ctx* c, int exhaustive) {
     return CRUSH_OK;
 }
 
+int crush_set_barrier_polls(crush_ctx* c, int polls) {
+    if (!c || polls < 0) return crush::fail(CRUSH_ERR_INVALID, "polls must be >= 0");
+    c->res_polls = polls;
+    return CRUSH_OK;
+}
+
 int crush_set_step_fusion(crush_ctx* c, int fused) {
     if (!c || (fused != 0 && fused != 1)) return crush::fail(CRUSH_ERR_INVALID, "fused must be 0 or 1");
     c->tuning_fixed = true;
@@ -3860,6 +3886,8 @@ int crush_contact_search_stats(crush_ctx* c, int id, uint64_t* out, int reset) {
 
 int crush_run_state(crush_ctx* c, double* u, double* v) {
     if (!c) return crush::fail(CRUSH_ERR_INVALID, "null context");
+    const int st = resident_outcome(c);
+    if (st != CRUSH_OK) return st;
     if (u) CK(cudaMemcpyAsync(u, c->u, sizeof(double) * 3 * c->n_nodes, cudaMemcpyDeviceToHost, c->stream));
     if (v) CK(cudaMemcpyAsync(v, c->v, sizeof(double) * 3 * c->n_nodes, cudaMemcpyDeviceToHost, c->stream));
     return sync(c);

@@ -2377,7 +2377,9 @@ cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks) {
         const cudaError_t e = allow_resident_smem(kernel, threads, a.el.n_sc > 0);
         if (e != cudaSuccess) return e;
     }
-    return cudaLaunchCooperativeKernel(kernel, grid, tpb, args, smem, s);
+    const cudaError_t e = cudaLaunchCooperativeKernel(kernel, grid, tpb, args, smem, s);
+    if (e == cudaSuccess) k_steps_failed<<<(unsigned)blocks, TPB, 0, s>>>(a.sync, a.ca[0], a.n_slaves);
+    return e;
 }
 void launch_node_cn(cudaStream_t s, const uint32_t* cnode, long long i0, long long i1, uint32_t* node_cn) {
     if (i1 > i0) k_node_cn<<<(unsigned)blocks_for(i1 - i0, TPB), TPB, 0, s>>>(cnode, i0, i1, node_cn);

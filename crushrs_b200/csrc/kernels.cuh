@@ -419,10 +419,11 @@ void launch_frames(cudaStream_t s, const FrameArrays& f, const double* u, const 
 
 // ---- Resident step kernel (resident.cuh) ----
 struct ResidentSync {
-    unsigned count, gen;  // grid barrier: arrivals, barriers with a serial part passed
-    int error;            // a block gave up waiting at a barrier
-    int pad;
+    unsigned count, gen;  // grid barrier: arrivals, barriers with a serial part passed (cleared for every launch)
+    int error;            // a block gave up waiting at a barrier (cleared when a run begins, as the next)
+    int dead;             // a launch before this one gave up
 };
+constexpr int RESIDENT_POLLS = 1 << 22;   // of a barrier before a block gives up (about 3 s), unless the caller sets another limit
 constexpr int RESIDENT_MAX_SLOTS = 1024;  // crashes of one launch (their control views are in shared memory)
 struct ResidentArgs {
     ElementArrays el;     // el_run
@@ -439,6 +440,7 @@ struct ResidentArgs {
     long long step0;
     int n_steps;
     int adaptive, check_steps, any_separation, hist_on;
+    int polls;            // of a barrier before a block gives up
     long long n_slaves;
     long long n_busy;     // honeycomb elements of the crashes not known to be done
     int contact0;         // first contact of those crashes (the ones before it are done)
@@ -449,7 +451,9 @@ struct ResidentArgs {
     int chunk_off[ACTIVE_SPACES + 1];  // the spaces' chunks that hold entities, numbered one after the other
 };
 // Steps [step0, step0 + n_steps) of every slot in one cooperative launch of
-// `blocks` blocks (at most resident_blocks: those that fit the device at once).
+// `blocks` blocks (at most resident_blocks: those that fit the device at once),
+// and the clean-up behind it in case it gave up: RESIDENT_LAUNCHES kernels.
+constexpr int RESIDENT_LAUNCHES = 2;
 int resident_blocks(int device, int n_sms);
 cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks);
 // node_cn of contact nodes [i0, i1).

@@ -33,22 +33,21 @@
 constexpr int RES_SMALL = 256, RES_LARGE = 512;
 constexpr int RES_ST_LANES = 4;       // lanes per static-grid entry (as many as emit a hit's events)
 constexpr int RES_GRID_LANES = 32;    // lanes per dynamic-grid entry
-// Polls of a barrier before a block gives up (about 3 s): the run then ends
-// with a timeout status instead of a hang.
-constexpr int RES_SPIN_LIMIT = 1 << 22;
-
 // Grid barrier: every block adds one to `count` and waits until all have.
 // With a serial part, the last block to arrive runs it, with everything the
 // others wrote before it visible, and lets them go by `gen`. Without one, the
 // blocks watch the count itself, a round trip less. False when a block gave up
 // waiting: every block then leaves the kernel (those that did not see it give
-// up at their next barrier).
+// up at their next barrier, which the ones that left never reach). A barrier
+// that some block passed had every block arrive, so a launch that gives up
+// leaves one phase half done and nothing of the next.
 struct ResidentBarrier {
     ResidentSync* y;
+    int limit;  // polls before a block gives up
     unsigned target, gen;
 
     __device__ __forceinline__ int wait(const unsigned* word, unsigned want) {
-        for (int polls = 0; polls < RES_SPIN_LIMIT; ++polls) {
+        for (int polls = 0; polls < limit; ++polls) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
             if ((int)(v - want) >= 0) return 1;
@@ -410,7 +409,8 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
     // the next search's. None without an entry to look up (bodies that miss
     // each other, or start apart by more than the contact's reach).
     const bool cells = grids && A.ca[0].n_buckets > 0;
-    ResidentBarrier barrier{A.sync, 0, 0};
+    ResidentBarrier barrier{A.sync, A.polls, 0, 0};
+    if (A.sync->dead) return;  // an earlier launch of the run gave up
     // emitted: the search emitted this step's events. pending_end: the last
     // step's end is still to be written to the control blocks. pending_record:
     // a record's partial sums are still to be added up.
@@ -725,5 +725,23 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
         deal.base = 0;
         record_sums(deal);
         barrier(&s_state, record_close);
+    }
+}
+
+// Behind every launch of k_steps: after one that gave up, the bookkeeping that
+// a contact search expects clear, which its half-done phase may have left set
+// (grid counts, event lists, big-face hits); the run's later launches then
+// return at once.
+__global__ void k_steps_failed(ResidentSync* y, ContactArrays ca, long long n_slaves) {
+    if (!y->error) return;
+    y->dead = 1;
+    const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = (long long)gridDim.x * blockDim.x;
+    if (ca.n_contacts == 0) return;
+    for (long long i = i0; i < ca.n_buckets; i += n) ca.counts[i] = 0;
+    for (long long i = i0; i < ca.n_cnodes; i += n) ca.ev_count[i] = 0;
+    for (long long i = i0; i < n_slaves; i += n) ca.big_best[i] = BIG_NONE;
+    if (i0 == 0) {
+        *ca.ev_pool_n = 0;
+        *ca.gather_count = 0;
     }
 }

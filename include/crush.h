@@ -257,6 +257,12 @@ int crush_contact_search_stats(crush_ctx* ctx, int contact_id, uint64_t* out, in
  * Both give the same hits: the grids only skip faces that cannot pass the
  * narrow test. For checking that equality; takes effect at the next step. */
 int crush_set_contact_search(crush_ctx* ctx, int exhaustive);
+/* How often a block of the resident step kernel polls a barrier before it
+ * gives up (4194304, about 3 s, unless set; 0 gives up at once). Every block
+ * then leaves, the run's remaining steps do nothing, and the calls that read
+ * the run return CRUSH_ERR_TIMEOUT until crush_run_begin. Takes effect at the
+ * next issue of steps. No counterpart in the reference. */
+int crush_set_barrier_polls(crush_ctx* ctx, int polls);
 /* fused = 1 runs a step whose next step starts with no stable-dt
  * check, record or reduction stop rule as one pass over the nodes (the
  * step's full update and the next step's half step), with the next step's
