@@ -3816,6 +3816,12 @@ int crush_frame_get(crush_ctx* c, int slot, int64_t frame, double* time, int64_t
 
 int crush_get_tuning(const crush_ctx* c, crush_tuning* out) {
     if (!c || !out) return crush::fail(CRUSH_ERR_INVALID, "null argument");
+    if (c->run_open && !c->tuned && !c->tuning_fixed) {
+        // a run that began with resident steps has not needed the lanes so far
+        CK(cudaSetDevice(c->device));
+        const int st = autotune(const_cast<crush_ctx*>(c));
+        if (st != CRUSH_OK) return st;
+    }
     std::memset(out, 0, sizeof(*out));
     out->slave_lanes = c->slave_lanes;
     out->forces_schedule = c->forces_schedule;

@@ -352,10 +352,13 @@ int crush_resample(const double* t, const double* y, int64_t n, double t0, doubl
                    int64_t cap, int64_t* n_out);
 
 /* Launch schedule of a context, chosen by the engine's autotuner (no
- * counterpart in the reference). The first crush_run_begin of a context times
- * the run's contact pass with 1, 2, 4, 8, 16 and 32 lanes per primary-node search
- * on the context's own models and keeps the fastest; all choices find the
- * same hits. */
+ * counterpart in the reference). Before its first step that is a launch
+ * sequence (or when crush_get_tuning asks for it, in an open run), a context
+ * times the run's contact pass with 1, 2, 4, 8, 16 and 32 lanes per
+ * primary-node search on its own models and keeps the fastest; all choices
+ * find the same hits. Small contexts step in the resident step kernel, which
+ * has no schedule to choose, until crush_set_tuning or crush_set_step_fusion
+ * fixes one. */
 typedef struct crush_tuning {
     int32_t slave_lanes;         /* lanes per primary-node search */
     int32_t forces_schedule;     /* element kernel: 0 one persistent wave of blocks taking chunks from a queue,
@@ -371,7 +374,8 @@ typedef struct crush_tuning {
                                     steps with 2 / 1; 0 = not measured */
 } crush_tuning;
 /* Re-tune now, at the open run's current state (e.g. late in a crash, when
- * crushed faces change the search); the next step uses the new schedule.
+ * crushed faces change the search); the next step that is a launch sequence
+ * uses the new schedule.
  * The step schedule is tuned on the run's own steps: a run of a context of
  * 2,000,000+ hexahedra times six candidates (separate steps leaving 8 or 16
  * SMs of the element kernel's wave to the side streams, with or without the
@@ -380,6 +384,9 @@ typedef struct crush_tuning {
  * the fastest; smaller contexts take separate steps with 8 SMs left free.
  * The contact lanes are re-tuned every 1000 steps. */
 int crush_autotune(crush_ctx* ctx, crush_tuning* out);
+/* The schedule and its measured times. In an open run whose steps have all
+ * been resident ones, the lanes are tuned by this call, at the run's current
+ * state (which it does not change). */
 int crush_get_tuning(const crush_ctx* ctx, crush_tuning* out);
 /* Fixes the schedule to t's slave_lanes, forces_schedule,
  * fused_contact_side and early_contact (measured fields ignored) and turns automatic tuning off for this context. Every
@@ -390,8 +397,9 @@ int crush_set_tuning(crush_ctx* ctx, const crush_tuning* t);
  *
  * No counterpart in the reference, whose unit of work is one model per
  * process (src/bin/crushrs.rs:30). A batch context holds n models ("slots")
- * resident on one GPU; every step is one launch sequence over the nodes and
- * elements of all slots, and each slot carries its own device control block
+ * resident on one GPU; every step is one pass over the nodes and elements of
+ * all slots (a launch sequence, or a step of the resident step kernel while
+ * the slots still running are few or small), and each slot carries its own device control block
  * (time, step, stable dt, mass scaling, stop rule), so slots of different
  * sizes and step sizes advance together and each stops on its own rule. The
  * arithmetic of every slot is the arithmetic of the same model run alone:
