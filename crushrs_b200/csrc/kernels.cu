@@ -2729,11 +2729,18 @@ void launch_contact_geometry(cudaStream_t s, const ContactArrays& ca, const Node
 namespace crush {
 namespace {
 
-// Four launches: faces and filter box, search and forces, sums, stores. A call
-// is bound by their latency (a chain of reads in each, one warp's instruction
-// stream): 304 faces and 120 nodes take 33.8 us; a box, a compaction of
-// the hits in blocks of their own and faces tested 32 at a time to the end took
-// 56.3 us in six launches.
+// Four launches: faces and filter box, search and forces, sums, stores. A small
+// call is bound by their latency (a chain of reads in each, one warp's instruction
+// stream), a large one by the box tests of every entry on every face. The boxes
+// are kept as planes of their own, so that a warp's 32 faces are two lines a
+// plane: read from the faces' 192-byte records they took 32 lines each, and large
+// calls were slower than testing one box side after the other. Primary entries
+// on a plate of 304, 4096 and 16,384 faces, in us (none of them hit; from records
+// with every block scanning all entries for hits / as here):
+//   120 entries      23 /  21      50 /  35     149 /  86
+//   2000             35 /  23     135 /  39     498 /  92
+//   16,384          138 /  41     977 / 132    3824 / 469
+// and with every entry a hit 30 / 31, 152 / 150, 1085 / 1092 us on 304 faces.
 constexpr int STATIC_TPB = 128;
 constexpr int STATIC_SEARCH_TPB = 64;
 constexpr int STATIC_TILE = STATIC_TPB;
@@ -2799,6 +2806,8 @@ __global__ void __launch_bounds__(STATIC_FACE_TPB) k_static_faces(StaticContactS
                 }
                 g.lo[d] = lo + -md;
                 g.hi[d] = hi + md;
+                sc->face_box[d][f] = g.lo[d];
+                sc->face_box[3 + d][f] = g.hi[d];
             }
             sc->geo[f] = g;
         }
@@ -2823,6 +2832,8 @@ __global__ void __launch_bounds__(STATIC_FACE_TPB) k_static_faces(StaticContactS
             sc->pen_max_bits = 0;
         }
     }
+    if (blockIdx.x == 0)
+        for (long long w = threadIdx.x; 32 * w < n_nodes; w += blockDim.x) sc->hit_mask[w] = 0;
 }
 
 // Warp per primary-node entry: the filter, then the smallest face index that
@@ -2868,9 +2879,9 @@ __global__ void __launch_bounds__(STATIC_SEARCH_TPB) k_static_search(StaticConta
         bool in[STATIC_BATCH];
 #pragma unroll
         for (int k = 0; k < STATIC_BATCH; ++k) {
-            const long long f = f0 + 32 * k + lane;
-            const FaceGeo& g = sc->geo[f < n_faces ? f : 0];
-            const double l0 = g.lo[0], l1 = g.lo[1], l2 = g.lo[2], h0 = g.hi[0], h1 = g.hi[1], h2 = g.hi[2];
+            const long long f = f0 + 32 * k + lane, q = f < n_faces ? f : 0;
+            const double l0 = sc->face_box[0][q], l1 = sc->face_box[1][q], l2 = sc->face_box[2][q];
+            const double h0 = sc->face_box[3][q], h1 = sc->face_box[4][q], h2 = sc->face_box[5][q];
             in[k] = f < n_faces && !(p[0] < l0 || p[0] > h0 || p[1] < l1 || p[1] > h1 || p[2] < l2 || p[2] > h2);
         }
         int count = 0;
@@ -2894,11 +2905,7 @@ __global__ void __launch_bounds__(STATIC_SEARCH_TPB) k_static_search(StaticConta
         first = __reduce_min_sync(0xffffffffu, best);
         if (first != INT_MAX) sd = __shfl_sync(0xffffffffu, best_sd, __ffs(__ballot_sync(0xffffffffu, best == first)) - 1);
     }
-    if (lane != 0) return;
-    if (first == INT_MAX) {
-        sc->hit[s] = -1;
-        return;
-    }
+    if (lane != 0 || first == INT_MAX) return;
     const double scale = node_scale ? node_scale[s] : 1.0;
     const double m = masses[n];
     const double depth = fmin(-sd, 0.1 * md);
@@ -2906,6 +2913,7 @@ __global__ void __launch_bounds__(STATIC_SEARCH_TPB) k_static_search(StaticConta
     const double mag = fmin(k_pen * depth, m * 1.0e5);
     const FaceGeo& g = sc->geo[first];
     sc->hit[s] = first;
+    atomicOr(&sc->hit_mask[s >> 5], 1u << (s & 31));
     sc->hit_force[3 * s] = mag * g.n[0];
     sc->hit_force[3 * s + 1] = mag * g.n[1];
     sc->hit_force[3 * s + 2] = mag * g.n[2];
@@ -2917,46 +2925,72 @@ __global__ void __launch_bounds__(STATIC_SEARCH_TPB) k_static_search(StaticConta
 // corners): the node's force value after this contact, adding the hits in
 // entry order — +F for its own hit, -F/4 per corner it fills on a hit face —
 // starting from the value in f_accum (src/contact.rs:146-153).
-// The hits are listed in entry order by each block for itself, a tile of
-// entries at a time.
+// The hits are numbered in entry order by each block for itself: a thread per
+// 128 entries counts the bits of their mask, and the block takes the hits a
+// tile at a time.
 __global__ void __launch_bounds__(STATIC_TPB) k_static_occ(StaticContactScratch* sc, int parts, long long n_nodes,
                                                            const uint32_t* __restrict__ nodes, long long n_faces,
                                                            const uint32_t* __restrict__ faces, const double* __restrict__ f_accum) {
     __shared__ uint32_t t_node[STATIC_TILE];
     __shared__ uint4 t_face[STATIC_TILE];
     __shared__ double t_f[STATIC_TILE][3];
-    __shared__ int s_warp[STATIC_TPB / 32];
-    static_assert(STATIC_TILE == STATIC_TPB, "an entry per thread");
+    __shared__ uint32_t s_mask[STATIC_TPB][4];
+    __shared__ int s_before[STATIC_TPB], s_warp[STATIC_TPB / 32];
+    static_assert(STATIC_MAX_NODES <= 128 * STATIC_TPB && STATIC_TPB == STATIC_TILE, "a thread per 128 entries, a hit of a tile per thread");
     if (static_bad(sc, parts)) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long n_occ = n_nodes + 4 * n_faces;
     const long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = o < n_occ;
-    const long long n = live ? (long long)(o < n_nodes ? nodes[o] : faces[o - n_nodes]) : 0;
+    const long long n = live ? (o < n_nodes ? nodes[o] : faces[o - n_nodes]) : 0;
     double v0 = 0.0, v1 = 0.0, v2 = 0.0;
     if (live) {
         v0 = f_accum[3 * n];
         v1 = f_accum[3 * n + 1];
         v2 = f_accum[3 * n + 2];
     }
-    for (long long s0 = 0; s0 < n_nodes; s0 += STATIC_TILE) {
-        const long long s = s0 + threadIdx.x;
-        const int fc = s < n_nodes ? sc->hit[s] : -1;
-        const unsigned ballot = __ballot_sync(0xffffffffu, fc >= 0);
-        if (lane == 0) s_warp[w] = __popc(ballot);
-        __syncthreads();
-        int at = 0, nt = 0;
+    const int groups = (int)((n_nodes + 127) / 128);
+    int count = 0;
 #pragma unroll
-        for (int k = 0; k < STATIC_TPB / 32; ++k) {
-            const int c = s_warp[k];
-            at += k < w ? c : 0;
-            nt += c;
-        }
-        if (fc >= 0) {
-            at += __popc(ballot & ((1u << lane) - 1u));
-            t_node[at] = nodes[s];
-            t_face[at] = make_uint4(faces[4ll * fc], faces[4ll * fc + 1], faces[4ll * fc + 2], faces[4ll * fc + 3]);
-            for (int d = 0; d < 3; ++d) t_f[at][d] = sc->hit_force[3 * s + d];
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t m = 128ll * threadIdx.x + 32 * k < n_nodes ? sc->hit_mask[4 * threadIdx.x + k] : 0u;
+        s_mask[threadIdx.x][k] = m;
+        count += __popc(m);
+    }
+    int incl = count;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += y;
+    }
+    if (lane == 31) s_warp[w] = incl;
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int k = 0; k < STATIC_TPB / 32; ++k) {
+        incl += k < w ? s_warp[k] : 0;
+        total += s_warp[k];
+    }
+    s_before[threadIdx.x] = incl - count;
+    __syncthreads();
+    for (int h0 = 0; h0 < total; h0 += STATIC_TILE) {
+        const int nt = min(STATIC_TILE, total - h0);
+        if ((int)threadIdx.x < nt) {
+            // hit h: in the last group that starts at or before it, then its bit
+            const int h = h0 + threadIdx.x;
+            int lo = 0, hi = groups - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (s_before[mid] <= h) lo = mid;
+                else hi = mid - 1;
+            }
+            int r = h - s_before[lo], k = 0;
+            for (; k < 3 && r >= __popc(s_mask[lo][k]); ++k) r -= __popc(s_mask[lo][k]);
+            const long long s = 128ll * lo + 32 * k + (int)__fns(s_mask[lo][k], 0, r + 1);
+            const long long fc = sc->hit[s];
+            t_node[threadIdx.x] = nodes[s];
+            t_face[threadIdx.x] = make_uint4(faces[4 * fc], faces[4 * fc + 1], faces[4 * fc + 2], faces[4 * fc + 3]);
+            for (int d = 0; d < 3; ++d) t_f[threadIdx.x][d] = sc->hit_force[3 * s + d];
         }
         __syncthreads();
         // Few hits touch a node: eight are compared at a time, and those that

@@ -329,9 +329,11 @@ constexpr int STATIC_MAX_PARTS = STATIC_MAX_FACES / STATIC_FACE_TPB;
 constexpr int STATIC_MAX_OCC = STATIC_MAX_NODES + 4 * STATIC_MAX_FACES;  // node occurrences
 struct StaticContactScratch {
     FaceGeo geo[STATIC_MAX_FACES];
+    double face_box[6][STATIC_MAX_FACES];  // lo xyz, hi xyz of the faces' boxes, a plane each
     double hit_force[3 * STATIC_MAX_NODES];
     double occ[3 * STATIC_MAX_OCC];    // new force value of the node of each occurrence
-    int hit[STATIC_MAX_NODES];         // face hit by each primary node entry, or -1
+    int hit[STATIC_MAX_NODES];         // face hit by each primary node entry that hit
+    alignas(16) uint32_t hit_mask[STATIC_MAX_NODES / 32];  // bit per primary node entry: it hit
     double part_box[6][STATIC_MAX_PARTS];  // per block of the face pass: its faces' reference box (lo xyz, hi xyz)
     int part_bad[STATIC_MAX_PARTS];    // per block: it met a node id out of range (nothing is written then)
     unsigned long long pen_count, pen_max_bits;

@@ -497,7 +497,7 @@ int crush_run_issue(crush_ctx* ctx, int64_t n_steps);
  * suits small and mid-size contacts.
  *
  * Memory: the call allocates nothing, host or device. Its scratch is one
- * fixed-size record (about 5.4 MB) in this library's static device memory,
+ * fixed-size record (about 6.4 MB) in this library's static device memory,
  * one copy per device. The call clears what it uses at its start, so nothing
  * needs zeroing by the caller. The FIRST call in each CUDA context resolves
  * the record's address (cudaGetSymbolAddress, which may load the library's
