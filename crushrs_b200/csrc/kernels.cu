@@ -441,13 +441,12 @@ __global__ void k_incidence_split(long long nn, const uint32_t* __restrict__ rel
 // ---------------------------------------------------------------------------
 // Element forces (src/kernel_simd.rs:300-491, one element per thread).
 //
-// Bound by memory latency at 16 warps per SM (128 registers, 2 x 256 threads;
-// the figures are of that persistent wave).
-// H streams through four registers instead of being held in 80, and gradients
-// and Γ are loaded where they are used, twice: the second read of these 224 B
-// comes from L1 (112 KB per SM in flight). A device force call on 278,640
-// elements takes 65.1 us, 67.9 us with everything held; held gradients and Γ
-// with H streamed 67.6 us.
+// H streams through four registers instead of being held in 80. Gradients and
+// Γ are needed twice. HOLD keeps these 224 bytes in registers and streams them
+// past L2 like the other planes: the next kernels of a step then find the
+// nodes' arrays in L2, which a mesh near L2's size would else have pushed out.
+// Without, they are read again where they are used, from L1 or L2, and the
+// registers go to loads in flight.
 // ---------------------------------------------------------------------------
 #ifndef FORCES_TPB
 #define FORCES_TPB 256
@@ -455,7 +454,7 @@ __global__ void k_incidence_split(long long nn, const uint32_t* __restrict__ rel
 #ifndef FORCES_MINB
 #define FORCES_MINB 2
 #endif
-template <class C>
+template <bool HOLD, class C>
 __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeArrays& nd, Control* ctls, const C* view, int respect_done,
                                             long long e) {
     if (e >= el.n_hc) return;
@@ -473,6 +472,9 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
     const uint32_t nid[8] = {__float_as_uint(c0.x), __float_as_uint(c0.y), __float_as_uint(c0.z), __float_as_uint(c0.w),
                              __float_as_uint(c1.x), __float_as_uint(c1.y), __float_as_uint(c1.z), __float_as_uint(c1.w)};
     const float4* geo = el.planes + P_GRAD * S + e;  // dN/dX and Γ
+    float4 held[HOLD ? 14 : 1];
+    const auto first = [&](int k) { return HOLD ? held[HOLD ? k : 0] = __ldcs(geo + k * S) : __ldg(geo + k * S); };
+    const auto again = [&](int k) { return HOLD ? held[HOLD ? k : 0] : __ldg(geo + k * S); };
     // F = Σ x_i ⊗ ∇N_i with x = (X + u) as f32; q = U Γ with u as f32.
     M3f f;
     float q[12];
@@ -480,7 +482,7 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
         float grad[24];
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
-            const float4 g = __ldg(geo + k * S);
+            const float4 g = first(k);
             grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
         }
 #pragma unroll
@@ -499,7 +501,7 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
             for (int a = 0; a < 3; ++a)
 #pragma unroll
                 for (int c = 0; c < 3; ++c) f.m[3 * a + c] = x[a] * grad[3 * i + c] + f.m[3 * a + c];
-            const float4 g4 = __ldg(geo + (6 + i) * S);
+            const float4 g4 = first(6 + i);
             const float gam[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
             for (int mode = 0; mode < 4; ++mode)
@@ -555,17 +557,17 @@ __device__ __forceinline__ void forces_body(const ElementArrays& el, const NodeA
                 if (j > i) rr[j] = h4[idx % 4] * q[i] + rr[j];
             }
     }
-    // f_i += rr Γᵀ, gradients and Γ read again (L1) instead of kept in registers
+    // f_i += rr Γᵀ
     float grad[24];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-        const float4 g = __ldg(geo + k * S);
+        const float4 g = again(k);
         grad[4 * k] = g.x; grad[4 * k + 1] = g.y; grad[4 * k + 2] = g.z; grad[4 * k + 3] = g.w;
     }
     float fo[24];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const float4 g4 = __ldg(geo + (6 + i) * S);
+        const float4 g4 = again(6 + i);
         const float gam[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
@@ -616,12 +618,13 @@ __device__ __forceinline__ void gather_node(const NodeArrays& nd, const float* _
 // time, so a block that starts late (its SM busy with other streams' work)
 // takes fewer chunks instead of finishing late; the last block to finish
 // (queue[1] counts them) sets both counters back to zero.
+template <bool HOLD>
 __global__ void __launch_bounds__(FORCES_TPB, FORCES_MINB) k_forces(ElementArrays el, NodeArrays nd, Control* ctls, int respect_done,
                                                                     unsigned* queue) {
     if (!queue) {
         FOR_ACTIVE(el.act_hc, el.n_hc, 1, g) {
             int lane;
-            forces_body(el, nd, ctls, ctls, respect_done, active_entity(el.act_hc, g, 1, &lane));
+            forces_body<HOLD>(el, nd, ctls, ctls, respect_done, active_entity(el.act_hc, g, 1, &lane));
         }
         return;
     }
@@ -635,7 +638,7 @@ __global__ void __launch_bounds__(FORCES_TPB, FORCES_MINB) k_forces(ElementArray
         if (item >= chunks) break;
         for (int t = threadIdx.x; t < CHUNK; t += FORCES_TPB) {
             int lane;
-            forces_body(el, nd, ctls, ctls, respect_done, active_entity(el.act_hc, item * CHUNK + t, 1, &lane));
+            forces_body<HOLD>(el, nd, ctls, ctls, respect_done, active_entity(el.act_hc, item * CHUNK + t, 1, &lane));
         }
     }
     if (threadIdx.x == 0) {
@@ -904,7 +907,7 @@ constexpr int SMALL_TPB = 64;
 __global__ void __launch_bounds__(SMALL_TPB) k_forces_small(ElementArrays el, NodeArrays nd, Control* ctls, int respect_done, int hc_blocks) {
     __shared__ double sh[SMALL_TPB / 8][OCT_SHARED];
     if ((int)blockIdx.x < hc_blocks) {
-        forces_body(el, nd, ctls, ctls, respect_done, (long long)blockIdx.x * SMALL_TPB + threadIdx.x);
+        forces_body<false>(el, nd, ctls, ctls, respect_done, (long long)blockIdx.x * SMALL_TPB + threadIdx.x);
         return;
     }
     const long long i = (long long)(blockIdx.x - hc_blocks) * (SMALL_TPB / 8) + threadIdx.x / 8;
@@ -2467,6 +2470,13 @@ void launch_init_state(cudaStream_t s, long long h_begin, long long n_hc, long l
     if (n_hc <= h_begin) return;
     k_init_state<<<(unsigned)blocks_for(n_hc - h_begin, TPB), TPB, 0, s>>>(h_begin, n_hc, stride, state);
 }
+// Elements from which k_forces reads gradients and Γ twice instead of holding
+// them (forces_body). Steps of the step graphs, in us, held / read twice: one
+// crash of some 119,000 elements 67 / 73, of 140,602 77.5 / 85.3, of 155,194
+// 78.5 / 91.6, of 200,949 98.6 / 103.5, of 278,960 119.1 / 121.7, of 500,240
+// 186.9 / 186.0, of 900,774 301 / 294; batches of 450,526 197.9 / 199.0, of
+// 621,504 251.6 / 249.1, of 1,055,557 396 / 387.
+constexpr long long FORCES_HOLD_MAX = 475000;
 // What k_forces_small takes: every element of a mesh (no active lists, nothing
 // beside it on other streams to leave SMs to) with at most 128 threads per SM
 // of elastic ones. Its 64-thread blocks retire one by one, where the
@@ -2494,8 +2504,11 @@ void launch_forces(cudaStream_t s, const ElementArrays& el, const NodeArrays& nd
     long long cap = (long long)(n_sms > 2 * free_sms ? n_sms - free_sms : n_sms) * FORCES_MINB;
     if (schedule == 1) cap = GRID_CAP * 4;
     unsigned* q = schedule == 1 ? nullptr : queue;
-    if (el.n_hc > 0)
-        k_forces<<<active_grid(el.n_hc, 1, FORCES_TPB, cap), FORCES_TPB, 0, s>>>(el, nd, ctls, respect_done, q);
+    if (el.n_hc > 0) {
+        const unsigned grid = active_grid(el.n_hc, 1, FORCES_TPB, cap);
+        if (el.n_hc < FORCES_HOLD_MAX) k_forces<true><<<grid, FORCES_TPB, 0, s>>>(el, nd, ctls, respect_done, q);
+        else k_forces<false><<<grid, FORCES_TPB, 0, s>>>(el, nd, ctls, respect_done, q);
+    }
     if (el.n_sc > 0)
         k_forces_scalar<<<active_grid(el.n_sc, 1, SC_TPB, GRID_CAP), SC_TPB, 0, s>>>(el, nd, ctls, respect_done);
 }

@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
         pending_record = false;
         deal(tasks(0, 1), [&](int t) {
             int l;
-            forces_body(el, nd, ctls, view, 1, entity(0, t, 1, &l));
+            forces_body<false>(el, nd, ctls, view, 1, entity(0, t, 1, &l));
         });
         if (ELASTIC && A.sc_oct)
             deal(tasks(8, 8), [&](int t) {
