@@ -164,6 +164,7 @@ struct Slot {
     int contact0 = 0, n_contacts = 0, vehicle0 = 0, n_vehicles = 0;
     int part0 = 0, n_parts = 0;  // the slot's parts in the concatenated part numbering
     long long hc0 = 0, n_hc = 0, sc0 = 0, n_sc = 0, face0 = 0, n_faces = 0;  // honeycomb, scalar and face ranges
+    long long n_searched = 0;    // primary-node entries that a step searches with a warp each (no static grid)
     double contact_dt = INF, stable = INF, dt_floor = 0.0, dt0 = 0.0;
 };
 
@@ -1484,6 +1485,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         } else {
             for (int e = slave_off[q]; e < slave_off[q + 1]; ++e) (st_grid ? stslaves : gslaves).push_back((uint32_t)e);
         }
+        if (!st_grid) slots[contact_slot[q] - S0].n_searched += slave_off[q + 1] - slave_off[q];
     }
     trace.mark("contact entry lists");
     // ---- vehicles: per slot its ranges, then the node lists filled in parallel ----
@@ -2897,27 +2899,37 @@ int schedule_trial(crush_ctx* c) {
     return st;
 }
 
-// Contexts up to this size step in the resident kernel; larger ones by the
-// step graphs, whose streaming kernels use more of the memory bandwidth (us per
-// step, resident and graph: one crash of 90,578 elements 57.0 and 60.9, of
-// 140,602 77.5 and 80.5, of 200,949 101.0 and 100.1, of 278,960 118.8 and
-// 115.1; batches of 71,869 44.2 and 54.3, of 132,540 83.1 and 102.8, of 230,770
-// 147.6 and 152.4).
-constexpr long long RESIDENT_MAX_ELEMENTS = 160000;
+// Contexts up to these sizes step in the resident kernel; larger ones by the
+// step graphs, whose streaming kernels use more of the memory bandwidth and
+// share a search between more threads than the resident grid has.
+// Steps in us, resident / graphs on their automatic schedule (the same case
+// differs by some 3 % from one context to the next): one crash of 79,948 elements
+// 52.9 / 55.7, of 120,036 68.3 / 67.7, of 140,602 79 / 77, of 155,194 90 / 87;
+// 8 crashes of 85,620 together 61 / 69, of 121,311 74 / 88; 32 of 124,848 76 / 81,
+// 48 of 152,808 99 / 90. Many small crashes have more entries to search than the
+// grid has warps: 400 of 28,000 elements and 10,350 entries 49.3 / 52.7, 128 of
+// 64,064 and 9,024 52 / 51.5, of 96,096 and 11,168 75 / 73, 400 of 84,800 and
+// 18,400 100 / 92.5.
+constexpr long long RESIDENT_MAX_ELEMENTS = 125000;
+constexpr long long RESIDENT_MAX_SEARCHED = 11000;  // entries searched by a warp each
 constexpr long long RESIDENT_MAX_STEPS = 1000;  // steps of one launch
 
-// Honeycomb elements of the slots that the last read of the done flags left
-// running, and the first of those slots.
-long long busy_elements(const crush_ctx* c, int* first) {
-    long long n = 0;
-    int f = -1;
+// The slots that the last read of the done flags left running.
+struct Running {
+    int first = -1;  // the first of them
+    long long elements = 0, nodes = 0, searched = 0;  // honeycomb elements, nodes, entries searched by a warp each
+};
+Running running(const crush_ctx* c) {
+    Running r;
     for (int k = 0; k < c->n_slots; ++k)
         if (k >= (int)c->done_h.size() || !c->done_h[k]) {
-            n += c->slots[k].n_hc;
-            if (f < 0) f = k;
+            const Slot& sl = c->slots[k];
+            if (r.first < 0) r.first = k;
+            r.elements += sl.n_hc;
+            r.nodes += sl.n_nodes;
+            r.searched += sl.n_searched;
         }
-    if (first) *first = f;
-    return n;
+    return r;
 }
 
 // Whether the context's steps run in the resident kernel: small, on the
@@ -2925,8 +2937,9 @@ long long busy_elements(const crush_ctx* c, int* first) {
 // The size is that of the crashes not known to be done (a serving context keeps
 // the finished ones; the kernel visits the others' chunks).
 bool resident(const crush_ctx* c) {
-    return c->res_blocks > 0 && !c->tuning_fixed && !c->profiling && !c->ca.exhaustive && !c->frames_on &&
-           busy_elements(c, nullptr) + c->n_sc_free <= RESIDENT_MAX_ELEMENTS && c->n_slots <= RESIDENT_MAX_SLOTS;
+    if (c->res_blocks == 0 || c->tuning_fixed || c->profiling || c->ca.exhaustive || c->frames_on || c->n_slots > RESIDENT_MAX_SLOTS) return false;
+    const Running r = running(c);
+    return r.elements + c->n_sc_free <= RESIDENT_MAX_ELEMENTS && r.searched <= RESIDENT_MAX_SEARCHED;
 }
 
 // The active chunk lists before steps that read them: a step at a multiple of
@@ -2969,9 +2982,10 @@ int resident_steps(crush_ctx* c, long long n) {
     a.any_separation = c->any_separation ? 1 : 0;
     a.hist_on = c->hist_on ? 1 : 0;
     a.n_slaves = c->n_slaves;
-    int first = -1;
-    a.n_busy = busy_elements(c, &first);
-    a.contact0 = first < 0 ? 0 : c->slots[first].contact0;
+    const Running r = running(c);
+    a.n_busy = r.elements;
+    a.n_tasks = r.nodes / 32 + r.searched;
+    a.contact0 = r.first < 0 ? 0 : c->slots[r.first].contact0;
     // One crash: every chunk, until it is done; more: those of running crashes.
     a.lists = c->n_slots > 1 ? c->ab.lists : nullptr;
     const long long ns[ACTIVE_SPACES] = {c->n_hc, c->n_all, c->n_nodes, c->ca.n_grid_slaves, c->ca.n_cnodes, c->ca.n_dyn_faces,

@@ -445,6 +445,7 @@ struct ResidentArgs {
     int polls;            // of a barrier before a block gives up
     long long n_slaves;
     long long n_busy;     // honeycomb elements of the crashes not known to be done
+    long long n_tasks;    // warp tasks of their nodes and searched entries
     int contact0;         // first contact of those crashes (the ones before it are done)
     int sc_oct;           // elastic elements on eight lanes each (set by the launcher)
     const int* lists;     // active chunk lists (ab.lists), or null: every chunk of every space

@@ -29,7 +29,7 @@
 #pragma once
 
 // Threads per block: 256 with up to 255 registers each while an element per
-// thread fits, else 512 with 128.
+// thread and a warp per searched entry fit, else 512 with 128 (launch_resident).
 constexpr int RES_SMALL = 256, RES_LARGE = 512;
 constexpr int RES_ST_LANES = 4;       // lanes per static-grid entry (as many as emit a hit's events)
 constexpr int RES_GRID_LANES = 32;    // lanes per dynamic-grid entry
