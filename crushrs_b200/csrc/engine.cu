@@ -18,6 +18,7 @@
 #include <thread>
 #include <atomic>
 #include <chrono>
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <array>
@@ -403,6 +404,69 @@ struct Stager {
 
 int stager_copy(Stager* st, void* dst, const void* src, size_t bytes) { return st->copy(dst, src, bytes); }
 
+// Contexts up to these sizes step in the resident kernel; larger ones by the
+// step graphs, whose streaming kernels use more of the memory bandwidth and
+// share a search between more threads than the resident grid has.
+// Steps in us, resident / graphs on their automatic schedule (the same case
+// differs by some 3 % from one context to the next): one crash of 79,948 elements
+// 52.9 / 55.7, of 120,036 68.3 / 67.7, of 140,602 79 / 77, of 155,194 90 / 87;
+// 8 crashes of 85,620 together 61 / 69, of 121,311 74 / 88; 32 of 124,848 76 / 81,
+// 48 of 152,808 99 / 90. Many small crashes have more entries to search than the
+// grid has warps: 400 of 28,000 elements and 10,350 entries 49.3 / 52.7, 128 of
+// 64,064 and 9,024 52 / 51.5, of 96,096 and 11,168 75 / 73, 400 of 84,800 and
+// 18,400 100 / 92.5.
+constexpr long long RESIDENT_MAX_ELEMENTS = 125000;
+constexpr long long RESIDENT_MAX_SEARCHED = 11000;  // entries searched by a warp each
+constexpr long long RESIDENT_MAX_STEPS = 250;  // steps of one launch (4-20 ms: what another stream's kernels may wait)
+
+// A resident launch holds every SM for as long as it runs, and the kernels of
+// another context's step graphs wait for it one after the other. So a context
+// that the resident kernel takes steps by graphs all the same while one that
+// it does not take is at work on the device: they share it kernel by kernel.
+// (1000 steps of 278,960 elements beside a thread that runs 1290-element crashes:
+// 136 ms alone, 380-530 ms beside resident steps, 180-215 ms so.) Contexts that are
+// all small keep to it: eight threads with a 1610-element crash each take 86 ms,
+// 194 ms as graphs. The bits of a run do not depend on its path.
+struct GraphWork {
+    std::atomic<const void*> by{nullptr};  // the context that last issued graph steps for want of another path
+    std::atomic<long long> until{0};       // until when it counts as at work (steady clock, ns)
+};
+constexpr int GRAPH_WORK_DEVICES = 64;
+GraphWork g_graph_work[GRAPH_WORK_DEVICES];
+constexpr long long GRAPH_WORK_NS = 5000000;  // from one issue to the next: reading results, admitting crashes
+GraphWork* graph_work(int device) { return device >= 0 && device < GRAPH_WORK_DEVICES ? &g_graph_work[device] : nullptr; }
+long long now_ns() { return std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch()).count(); }
+void graph_work_until(int device, const void* ctx, long long until) {
+    if (GraphWork* w = graph_work(device)) {
+        w->by.store(ctx);
+        w->until.store(until);
+    }
+}
+// While it lives, and GRAPH_WORK_NS on: the set-up, the begin of a run or a
+// wait for steps of a context that steps by graphs (with many kernels that the
+// host waits for, each behind a resident launch else).
+struct GraphWorkScope {
+    int device;
+    const void* ctx;
+    bool on;
+    GraphWorkScope(int device, const void* ctx, bool on) : device(device), ctx(ctx), on(on) {
+        if (on) graph_work_until(device, ctx, LLONG_MAX);
+    }
+    ~GraphWorkScope() {
+        if (on) graph_work_until(device, ctx, now_ns() + GRAPH_WORK_NS);
+    }
+};
+// The context has no more graph steps to run, or is going away.
+void graph_work_over(int device, const void* ctx) {
+    if (GraphWork* w = graph_work(device)) w->by.compare_exchange_strong(ctx, nullptr);
+}
+// Whether another context's graph steps are at work.
+bool graph_work_beside(int device, const void* ctx) {
+    const GraphWork* w = graph_work(device);
+    const void* by = w ? w->by.load() : nullptr;
+    return by && by != ctx && now_ns() < w->until.load();
+}
+
 }  // namespace
 
 struct crush_ctx {
@@ -707,6 +771,7 @@ struct crush_ctx {
         return st;
     }
     ~crush_ctx() {
+        graph_work_over(device, this);
         for (cudaGraphExec_t g : graphs)
             if (g) cudaGraphExecDestroy(g);
         for (cudaEvent_t e : prof_ev) cudaEventDestroy(e);
@@ -2103,6 +2168,10 @@ int create_impl(const crush_model_desc* const* descs, int n_desc, int device, cr
     if (n_desc <= 0 || !descs) return crush::fail(CRUSH_ERR_INVALID, "no models");
     c->device = device;
     CK(cudaSetDevice(device));
+    long long hexes = 0;
+    for (int k = 0; k < n_desc; ++k)
+        if (descs[k]) hexes += descs[k]->n_hexes;
+    GraphWorkScope work(device, c, hexes > RESIDENT_MAX_ELEMENTS);
     CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     CK(cudaDeviceGetAttribute(&c->n_sms, cudaDevAttrMultiProcessorCount, device));
 
@@ -2628,9 +2697,12 @@ Control initial_control(const Slot& sl) {
 }
 
 bool resident(const crush_ctx* c);
+bool resident_fits(const crush_ctx* c);
 
 int run_begin(crush_ctx* c) {
     const long long N = c->n_nodes;
+    c->done_h.clear();  // nothing of a run before counts as done
+    GraphWorkScope work(c->device, c, !resident_fits(c));
     drop_graphs(c);
     CK(cudaMemsetAsync(c->u, 0, sizeof(double) * 3 * N, c->stream));
     CK(cudaMemcpyAsync(c->v, c->v0, sizeof(double) * 3 * N, cudaMemcpyDeviceToDevice, c->stream));
@@ -2899,21 +2971,6 @@ int schedule_trial(crush_ctx* c) {
     return st;
 }
 
-// Contexts up to these sizes step in the resident kernel; larger ones by the
-// step graphs, whose streaming kernels use more of the memory bandwidth and
-// share a search between more threads than the resident grid has.
-// Steps in us, resident / graphs on their automatic schedule (the same case
-// differs by some 3 % from one context to the next): one crash of 79,948 elements
-// 52.9 / 55.7, of 120,036 68.3 / 67.7, of 140,602 79 / 77, of 155,194 90 / 87;
-// 8 crashes of 85,620 together 61 / 69, of 121,311 74 / 88; 32 of 124,848 76 / 81,
-// 48 of 152,808 99 / 90. Many small crashes have more entries to search than the
-// grid has warps: 400 of 28,000 elements and 10,350 entries 49.3 / 52.7, 128 of
-// 64,064 and 9,024 52 / 51.5, of 96,096 and 11,168 75 / 73, 400 of 84,800 and
-// 18,400 100 / 92.5.
-constexpr long long RESIDENT_MAX_ELEMENTS = 125000;
-constexpr long long RESIDENT_MAX_SEARCHED = 11000;  // entries searched by a warp each
-constexpr long long RESIDENT_MAX_STEPS = 1000;  // steps of one launch
-
 // The slots that the last read of the done flags left running.
 struct Running {
     int first = -1;  // the first of them
@@ -2932,15 +2989,17 @@ Running running(const crush_ctx* c) {
     return r;
 }
 
-// Whether the context's steps run in the resident kernel: small, on the
+// Whether the resident kernel takes the context's steps: small, on the
 // automatic schedule, with nothing between the steps but what that kernel does.
 // The size is that of the crashes not known to be done (a serving context keeps
 // the finished ones; the kernel visits the others' chunks).
-bool resident(const crush_ctx* c) {
+bool resident_fits(const crush_ctx* c) {
     if (c->res_blocks == 0 || c->tuning_fixed || c->profiling || c->ca.exhaustive || c->frames_on || c->n_slots > RESIDENT_MAX_SLOTS) return false;
     const Running r = running(c);
     return r.elements + c->n_sc_free <= RESIDENT_MAX_ELEMENTS && r.searched <= RESIDENT_MAX_SEARCHED;
 }
+
+bool resident(const crush_ctx* c) { return resident_fits(c) && !graph_work_beside(c->device, c); }
 
 // The active chunk lists before steps that read them: a step at a multiple of
 // 20 builds them itself, any other needs those of a step before it — which
@@ -3060,6 +3119,7 @@ int issue_steps(crush_ctx* c, long long n_steps) {
             c->last_was_graph = false;
         }
     }
+    if (!resident_fits(c)) graph_work_until(c->device, c, now_ns() + GRAPH_WORK_NS);
     return CRUSH_OK;
 }
 
@@ -3079,12 +3139,16 @@ int resident_outcome(crush_ctx* c) {
 // Whether every slot has finished (device flags read back; synchronises).
 int all_done(crush_ctx* c, int* done) {
     c->done_h.resize(c->n_slots);
-    CK(cudaMemcpyAsync(c->done_h.data(), c->slot_done, sizeof(int) * c->n_slots, cudaMemcpyDeviceToHost, c->stream));
+    {
+        GraphWorkScope work(c->device, c, c->run_open && !resident_fits(c));
+        CK(cudaMemcpyAsync(c->done_h.data(), c->slot_done, sizeof(int) * c->n_slots, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+    }
     const int st = resident_outcome(c);
     if (st != CRUSH_OK) return st;
-    CK(cudaStreamSynchronize(c->stream));
     int d = 1;
     for (int x : c->done_h) d &= x ? 1 : 0;
+    if (d || resident_fits(c)) graph_work_over(c->device, c);
     *done = d;
     return CRUSH_OK;
 }
