@@ -901,8 +901,11 @@ __global__ void __launch_bounds__(SC_TPB) k_forces_scalar(ElementArrays el, Node
 // Both kinds of a mesh in one launch: blocks [0, hc_blocks) take 64
 // honeycomb elements each, the rest 8 elastic ones on eight lanes each. Small
 // blocks spread a few elements over the SMs, and the elastic elements (a
-// road's 360 took a launch of their own behind the others) run beside them: a
-// force call on 1290 + 264 elements takes 6.1 us, 12.3 us in three launches.
+// road's few hundred took a launch of their own behind the others) run beside
+// them: a force call on 1290 + 320 elements takes 6.1 us with the gather behind
+// it, 12.3 us in three launches. 163 registers, the elastic branch's, so 12 warps
+// per SM: a large mesh is bound by the latency of its element loads
+// (278,640 elements: 61 us, 44 us at the copy rate).
 constexpr int SMALL_TPB = 64;
 __global__ void __launch_bounds__(SMALL_TPB) k_forces_small(ElementArrays el, NodeArrays nd, Control* ctls, int respect_done, int hc_blocks) {
     __shared__ double sh[SMALL_TPB / 8][OCT_SHARED];
@@ -1705,11 +1708,11 @@ __device__ __forceinline__ void record_hit(const ContactArrays& ca, long long s,
 // face the reference's in-order scan with `break` finds
 // (src/contact.rs:115-157). Lane 0 sets the node's big_best back to
 // BIG_NONE for the next search, also when its crash has stopped.
-template <int LANES, class C>
-__device__ __forceinline__ int contact_slave_body(const ContactArrays& ca, const NodeArrays& nd, const C* ctls, int c0, int c1,
+template <int LANES>
+__device__ __forceinline__ void contact_slave_body(const ContactArrays& ca, const NodeArrays& nd, const Control* ctls, int c0, int c1,
                                                    int run_mode, double dt_override, const double* __restrict__ masses, long long s,
-                                                   bool live, int lane, double* sd_out = nullptr) {
-    const C* ctl = nullptr;
+                                                   bool live, int lane) {
+    const Control* ctl = nullptr;
     bool reset_big = false;
     if (live) {
         const int c = ca.slave_contact[s];
@@ -1797,15 +1800,13 @@ __device__ __forceinline__ int contact_slave_body(const ContactArrays& ca, const
         if (ob < best) { best = ob; best_sd = osd; }
     }
     if (reset_big) ca.big_best[s] = BIG_NONE;
-    if (!live || lane != 0) return -1;
+    if (!live || lane != 0) return;
     if (best == INT_MAX) {
         ca.hit[s] = -1;
-        return -1;
+        return;
     }
     ca.hit[s] = best;
     ca.hit_sd[s] = best_sd;
-    if (sd_out) *sd_out = best_sd;
-    return best;  // lane 0's: the face index, or -1
 }
 
 // run: the entries of `list` (grid_slaves or st_slaves, over their active
@@ -2482,14 +2483,18 @@ void launch_init_state(cudaStream_t s, long long h_begin, long long n_hc, long l
 // 621,504 251.6 / 249.1, of 1,055,557 396 / 387.
 constexpr long long FORCES_HOLD_MAX = 475000;
 // What k_forces_small takes: every element of a mesh (no active lists, nothing
-// beside it on other streams to leave SMs to) with at most 128 threads per SM
-// of elastic ones. Its 64-thread blocks retire one by one, where the
-// persistent wave's chunks of 256 end unevenly. Force call, k_forces and
-// k_forces_scalar behind it against k_forces_small: 13.2 and 7.1 us at 19,500
-// elements, 22.9 and 18.0 at 75,000, 34.2 and 28.3 at 130,000, 65.6 and 61.1
-// at 278,640.
+// beside it on other streams to leave SMs to) with few elastic ones. Its
+// 64-thread blocks retire one by one, where the persistent wave's chunks of 256
+// end unevenly. Force call, k_forces and k_forces_scalar behind it against
+// k_forces_small: 13.2 and 7.1 us at 19,500 elements, 22.9 and 18.0 at 75,000,
+// 34.2 and 28.3 at 130,000, 65.6 and 61.1 at 278,640. Elastic elements on eight
+// lanes cost eight threads each: calls issued one after the other take 35.0 and
+// 18.6 us with 2,312 of them beside 2,048 honeycomb ones, 35.2 and 31.1 with 14,408
+// beside 2,016, 37.4 and 43.2 with 26,608 beside 3,794. The line is on the safe
+// side of that.
+constexpr long long SMALL_ELASTIC_MAX = 2368;
 bool small_forces(const ElementArrays& el) {
-    return !el.act_hc.list && !el.sc_list && el.n_sc == el.sc_count && 8 * el.n_sc <= 148 * 128;
+    return !el.act_hc.list && !el.sc_list && el.n_sc == el.sc_count && el.n_sc <= SMALL_ELASTIC_MAX;
 }
 void launch_forces(cudaStream_t s, const ElementArrays& el, const NodeArrays& nd, Control* ctls, int respect_done, int n_sms,
                    int schedule, unsigned* queue) {

@@ -60,7 +60,7 @@ struct ResidentBarrier {
         asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(k) : "l"(&y->count) : "memory");
         return k;
     }
-    __device__ __forceinline__ bool operator()(int* s_state) {
+    __device__ __forceinline__ bool operator()() {
         __syncthreads();
         target += gridDim.x;
         int ok = 1;
@@ -263,8 +263,6 @@ __device__ __forceinline__ void resident_full(const ElementArrays& el, const Nod
     }
 }
 
-// ELASTIC: the context has elastic elements with a free node; without, their
-// code stays out of the kernel.
 // A static-grid entry by RES_ST_LANES lanes: nothing outside the union of the
 // fixed faces' key boxes, else the faces of its point's bucket, smallest first
 // (contact_slave_body's static part). Every lane of the warp calls; the face, or
@@ -384,6 +382,8 @@ __device__ __forceinline__ int resident_grid(const ContactArrays& ca, const Node
     *sd_out = best_sd;
     return best;
 }
+// ELASTIC: the context has elastic elements with a free node; without, their
+// code stays out of the kernel.
 template <int RES_TPB, bool ELASTIC>
 __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ ResidentArgs A) {
     __shared__ HeavyShared heavy;
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                     int l;
                     mass_scaling_body(el, nd, view, 0, entity(2, t, 1, &l));
                 });
-            if (!(go = barrier(&s_state))) break;
+            if (!(go = barrier())) break;
             deal.base = 0;
         }
 
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             if (pending_end) end_step(ended, false);
         }
         pending_end = false;
-        if (!(go = barrier(&s_state))) break;
+        if (!(go = barrier())) break;
         deal.base = 0;
 
         // Element forces and the moving faces' geometry.
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                 const long long k = entity(5, t, 1, &l);
                 contact_face_body<1>(ca, nd, view, 0, ca.dyn_faces, ca.n_dyn_faces, 1, 0, k, l);
             });
-        if (!(go = barrier(&s_state))) break;
+        if (!(go = barrier())) break;
         deal.base = 0;
 
         // Full update beside the search of the next step's contacts.
@@ -634,14 +634,14 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                 deal((int)((ca.n_buckets - ca.tab_off[A.contact0] + 31) / 32),
                      [&](int t) { grid_alloc_body(ca, A.contact0, ca.n_contacts, (long long)t * 32 + lane); });
                 contact_big_block(ca, nd, big_face, big_box);
-                if (!(go = barrier(&s_state))) break;
+                if (!(go = barrier())) break;
                 deal.base = 0;
                 deal(tasks(5, 32), [&](int t) {
                     int l;
                     const long long k = entity(5, t, 32, &l);
                     contact_insert_body(ca, 0, ca.dyn_faces, ca.n_dyn_faces, k, l);
                 });
-                if (!(go = barrier(&s_state))) break;
+                if (!(go = barrier())) break;
                 deal.base = 0;
             }
             deal(tasks(3, RES_GRID_LANES), [&](int t) {
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             });
         }
         if (sep) {
-            if (!(go = barrier(&s_state))) break;
+            if (!(go = barrier())) break;
             for (int k = blockIdx.x; summing && k < A.va.n_vehicles * A.va.vx_blocks; k += gridDim.x) {
                 vehicle_vx_block(A.va, nd.mass, nd.v, ctls, k, &heavy.sf[0][0], &heavy.sf[0][0] + VEH_TPB);
                 heavy_sync();
@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
         // otherwise the control blocks decide, with the next step's stable-dt
         // decision and chunk lists.
         if (plain) {
-            if (!(go = barrier(&s_state))) break;
+            if (!(go = barrier())) break;
             for (int sl = threadIdx.x; sl < n_slots; sl += RES_TPB) {
                 ControlView c = view[sl];
                 if (c.done) continue;
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
                 if (hist_due(A.hist, view + slot, slot, HIST_STEP) && r < A.hist.slot_max[slot]) hist_node(A.hist, nd, nd.f_ext, j, r);
             });
             pending_record = true;
-            if (!(go = barrier(&s_state))) break;
+            if (!(go = barrier())) break;
         }
         if (n_running == 0) break;
     }
