@@ -352,7 +352,7 @@ def batched_section(n, plain_sample, oracle_sample, device, world=1):
     if times:
         plain_s = statistics.median(times)
         out["plain"] = {"crashes_per_s": 1.0 / plain_s, "median_s_per_crash": plain_s, "sample": plain_sample,
-                        "path": "crush_create + crush_run per crash (CUDA graphs of 20 steps)"}
+                        "path": "crush_create + crush_run per crash (resident steps: one launch per 250)"}
         out["speedup_vs_plain"] = batched_cps * plain_s
         out["one_shot"]["speedup_vs_plain"] = n / (t4 - t2) * plain_s
         out["batched_equals_plain"] = bool(same)
