@@ -2647,6 +2647,7 @@ int rebuild_history(crush_ctx* c) {
     h.steps = steps;
     h.max_rec = stride;
     h.n_pu = (int)pu_slot.size();
+    for (int p = 0; p < h.n_pu; ++p) h.any_long |= pu_off[p + 1] - pu_off[p] > (uint32_t)HIST_LONG ? 1 : 0;
     h.n_an = (int)an_node.size();
     const size_t mark = c->allocs.size();
     auto up = [&](auto** dst, const auto& v) { return c->upload_const(dst, v); };

@@ -9,16 +9,22 @@ namespace {
 
 constexpr int HIST_TPB = 256;
 
-// Warp per (part unit, chunk): the chunk's sums into partial[pu][chunk].
+// Warp per (part unit, chunk): the chunk's sums into partial[pu][chunk]; where
+// a context has long part units, a block per chunk of those (and of every
+// eighth of the others, for eight chunks).
 __global__ void __launch_bounds__(HIST_TPB) k_hist_parts(HistoryArrays h, NodeArrays nd, const Control* ctls,
                                                          const double* __restrict__ f_ext, int mode, const double* __restrict__ f_ext_odd) {
-    const int w = blockIdx.x * (HIST_TPB / 32) + (threadIdx.x >> 5);
-    const int pu = w / HIST_BLOCKS, b = w % HIST_BLOCKS;
-    if (pu >= h.n_pu) return;  // warp-uniform, as the next
+    __shared__ double sh[HIST_PART_VALUES * HIST_TREE];
+    static_assert(HIST_TPB == HIST_TREE && HIST_BLOCKS % (HIST_TPB / 32) == 0, "a column per thread, a block's chunks of one part");
+    const int first = h.any_long ? blockIdx.x : blockIdx.x * (HIST_TPB / 32);  // the block's first (part unit, chunk)
+    const int pu = first / HIST_BLOCKS, b = first % HIST_BLOCKS;
+    const bool is_long = h.any_long && hist_long(h, pu);
+    if (h.any_long && !is_long && b % (HIST_TPB / 32) != 0) return;  // block-uniform, as the next
     const int slot = h.pu_slot[pu];
     if (!hist_due(h, ctls + slot, slot, mode)) return;
     const bool odd = mode == HIST_FINAL && f_ext_odd && ((ctls[slot].step - 1) & 1);
-    hist_part_warp(h, nd, odd ? f_ext_odd : f_ext, pu, b, threadIdx.x & 31);
+    if (is_long) hist_part_block(h, nd, odd ? f_ext_odd : f_ext, pu, b, sh);
+    else hist_part_warp(h, nd, odd ? f_ext_odd : f_ext, pu, b + (threadIdx.x >> 5), threadIdx.x & 31);
 }
 
 // Block per slot: the record's part states (a warp per part), accelerometer
@@ -51,7 +57,9 @@ __global__ void __launch_bounds__(HIST_TPB) k_hist_finish(HistoryArrays h, NodeA
 
 void launch_history(cudaStream_t s, const HistoryArrays& h, const NodeArrays& nd, const Control* ctls, const double* f_ext, int mode,
                     const double* f_ext_odd) {
-    if (h.n_pu > 0) k_hist_parts<<<(unsigned)((h.n_pu * HIST_BLOCKS + HIST_TPB / 32 - 1) / (HIST_TPB / 32)), HIST_TPB, 0, s>>>(h, nd, ctls, f_ext, mode, f_ext_odd);
+    if (h.n_pu > 0)
+        k_hist_parts<<<(unsigned)(h.n_pu * HIST_BLOCKS / (h.any_long ? 1 : HIST_TPB / 32)), HIST_TPB, 0, s>>>(h, nd, ctls, f_ext, mode,
+                                                                                                          f_ext_odd);
     k_hist_finish<<<(unsigned)h.n_slots, HIST_TPB, 0, s>>>(h, nd, ctls, f_ext, mode, f_ext_odd);
 }
 

@@ -9,6 +9,7 @@ namespace crush {
 namespace {
 
 constexpr int HIST_TREE = 256;  // columns of the part sums' tree
+static_assert(HIST_LONG == HIST_BLOCKS * HIST_TREE, "a node per column");
 
 // Whether slot `slot` takes a record now: its run's first record, a step
 // that is a multiple of history_steps, or the last step of a finished crash;
@@ -138,6 +139,32 @@ __device__ __forceinline__ void hist_part_warp(const HistoryArrays& h, const Nod
 #pragma unroll
         for (int k = 0; k < HIST_PART_VALUES; ++k) o[k] = s.a[k];
     }
+}
+
+// The same sums by HIST_TREE threads, a column each, for the part units of
+// large meshes (more than HIST_LONG nodes): a warp's lanes would each add eight
+// columns of many nodes one after the other. `sh`: HIST_PART_VALUES x HIST_TREE
+// doubles. A step of 279,936 elements with a record takes 161 us, 259 us by
+// warps (126 without a record); of 55,566 elements 47 and 71 (38).
+__device__ __forceinline__ bool hist_long(const HistoryArrays& h, int pu) { return h.pu_off[pu + 1] - h.pu_off[pu] > (uint32_t)HIST_LONG; }
+__device__ __forceinline__ void hist_sync() { asm volatile("bar.sync 1, %0;" ::"n"(HIST_TREE) : "memory"); }
+__device__ __noinline__ void hist_part_block(const HistoryArrays& h, const NodeArrays& nd, const double* f_ext, int pu, int b, double* sh) {
+    const long long lo = h.pu_off[pu], len = (long long)h.pu_off[pu + 1] - lo;
+    const long long per = (len + HIST_BLOCKS - 1) / HIST_BLOCKS;
+    const long long i0 = lo + b * per, i1 = min(lo + len, i0 + per);
+    const HistSums s = hist_column(h, nd, f_ext, i0 + threadIdx.x, i1);
+#pragma unroll
+    for (int k = 0; k < HIST_PART_VALUES; ++k) sh[k * HIST_TREE + threadIdx.x] = s.a[k];
+    hist_sync();
+    const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x >> 5; k < HIST_PART_VALUES; k += HIST_TREE / 32) {
+        const double* c = sh + k * HIST_TREE + lane;
+        double x = ((c[0] + c[128]) + (c[64] + c[192])) + ((c[32] + c[160]) + (c[96] + c[224]));
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+        if (lane == 0) h.partial[((long long)pu * HIST_BLOCKS + b) * HIST_PART_VALUES + k] = x;
+    }
+    hist_sync();  // sh is free again
 }
 
 // Record r of part unit pu by one warp: lane k < HIST_PART_VALUES adds value k

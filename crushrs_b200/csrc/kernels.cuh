@@ -346,6 +346,7 @@ struct StaticContactScratch {
 // kernel adds in block order. Records are kept per slot in arrays of
 // max_rec entries.
 constexpr int HIST_BLOCKS = 32;
+constexpr int HIST_LONG = 8192;  // nodes of a part unit from which a block sums a chunk, not a warp
 constexpr int HIST_PART_VALUES = 11;  // mass, velocity 3, displacement 3, acceleration 3, kinetic energy
 constexpr int HIST_NODE_VALUES = 21;  // position, displacement, velocity, acceleration, local u, v, a (3 each)
 enum HistMode { HIST_INITIAL = 0, HIST_STEP = 1, HIST_FINAL = 2 };
@@ -358,6 +359,7 @@ struct HistoryArrays {
     const int* slot_pu_off;     // n_slots+1: the slot's part units
     const int* slot_an_off;     // n_slots+1: the slot's accelerometer nodes
     int n_pu;
+    int any_long;               // some part unit has more than HIST_LONG nodes
     const uint32_t* pu_off;     // n_pu+1 into pu_nodes
     const uint32_t* pu_nodes;   // global node ids
     const int* pu_slot;

@@ -397,6 +397,8 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
     constexpr int RES_WARPS = RES_TPB / 32;
     ControlView* view = reinterpret_cast<ControlView*>(oct_shared + (ELASTIC && A.sc_oct ? OCT_SHARED * RES_TPB / 8 : 0));
     static_assert(RES_TPB >= HEAVY_TPB && VEH_TPB == HEAVY_TPB && sizeof(heavy.sf) >= 2 * sizeof(double) * VEH_TPB, "block sums");
+    static_assert(RES_TPB >= HIST_TREE && sizeof(heavy) >= sizeof(double) * HIST_PART_VALUES * HIST_TREE && alignof(HeavyShared) >= 8,
+                  "a history's part sums");
     const bool summing = threadIdx.x < HEAVY_TPB;  // the threads of the block-wide sums
     const bool odd_jobs = blockIdx.x == gridDim.x - 1;  // the block that does what one block does
     const int lane = threadIdx.x & 31;
@@ -704,8 +706,14 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
             deal.base = 0;
             deal(A.hist.n_pu * HIST_BLOCKS, [&](int t) {
                 const int pu = t / HIST_BLOCKS, slot = A.hist.pu_slot[pu];
+                if (A.hist.any_long && hist_long(A.hist, pu)) return;
                 if (hist_due(A.hist, view + slot, slot, HIST_STEP)) hist_part_warp(A.hist, nd, nd.f_ext, pu, t % HIST_BLOCKS, lane);
             });
+            for (int t = blockIdx.x; A.hist.any_long && threadIdx.x < HIST_TREE && t < A.hist.n_pu * HIST_BLOCKS; t += gridDim.x) {
+                const int pu = t / HIST_BLOCKS, slot = A.hist.pu_slot[pu];
+                if (hist_long(A.hist, pu) && hist_due(A.hist, view + slot, slot, HIST_STEP))
+                    hist_part_block(A.hist, nd, nd.f_ext, pu, t % HIST_BLOCKS, reinterpret_cast<double*>(&heavy));
+            }
             deal((A.hist.n_an + 31) / 32, [&](int t) {
                 const int j = t * 32 + lane;
                 if (j >= A.hist.n_an) return;
