@@ -1430,10 +1430,15 @@ __device__ __forceinline__ int box_level(const ContactArrays& ca, int c, const d
 // is listed as a big face with its key box. Every face of a grid contact that
 // the pass visits gets its cell record (level -1: no inserts), so the fill
 // pass, over the same faces, inserts exactly what was counted.
-// One lane per face when no contact has a grid: the geometry is one chain that
-// more lanes only repeat (39,680 faces on the SMs the element kernel leaves: 77 us,
-// 158 us with four).
+// One lane per face when no contact has a grid and the faces are many: the
+// geometry is one chain that more lanes only repeat (39,680 faces on the SMs the
+// element kernel leaves: 77 us, 158 us with four). A few faces on one lane each
+// fill a few SMs only (882 faces: 24 us, 5 us with four), and an exhaustive search
+// waits for them. Steps with one / four lanes: 2040 faces 43.7 / 43.2 us, 4152 with
+// early contact forces 63.4 / 65.1, 8408 103.5 / 104.8, 39,800 351 / 364;
+// exhaustive 2040 77.5 / 56.8, 16,888 364 / 344, 39,800 776 / 777.
 constexpr int FACE_LANES = 4;
+constexpr long long FACES_ONE_LANE = 4000;
 template <int LANES, class C>
 __device__ __forceinline__ void contact_face_body(const ContactArrays& ca, const NodeArrays& nd, const C* ctls, int c0,
                                                   const uint32_t* __restrict__ face_list, long long n, int run_mode, int do_grid,
@@ -2613,9 +2618,9 @@ void launch_contact_search(cudaStream_t s, const ContactArrays& ca, const NodeAr
     // cursors, big-face list), whatever ran before it.
     cudaMemsetAsync(ca.grid_state, 0, sizeof(int) * (2 * (size_t)ca.contact_room + 1), s);
     if (n_list > 0) {
-        if (do_grid)
+        if (do_grid || ca.exhaustive || n_list < FACES_ONE_LANE)
             k_contact_faces<FACE_LANES><<<active_grid(n_list, FACE_LANES, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, ctls, c0, list,
-                                                                                                               n_list, run_mode, 1, act);
+                                                                                                               n_list, run_mode, do_grid, act);
         else
             k_contact_faces<1><<<active_grid(n_list, 1, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, ctls, c0, list, n_list, run_mode, 0,
                                                                                              act);
@@ -2733,8 +2738,12 @@ void launch_contact_geometry(cudaStream_t s, const ContactArrays& ca, const Node
     (void)f0;
     if (c1 <= c0 || n_faces <= 0) return;
     (void)c1;
-    k_contact_faces<1><<<active_grid(n_faces, 1, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, nullptr, c0, nullptr, n_faces, 0, 0,
-                                                                                      Active{nullptr, nullptr});
+    if (n_faces < FACES_ONE_LANE)
+        k_contact_faces<FACE_LANES><<<active_grid(n_faces, FACE_LANES, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(
+            ca, nd, nullptr, c0, nullptr, n_faces, 0, 0, Active{nullptr, nullptr});
+    else
+        k_contact_faces<1><<<active_grid(n_faces, 1, FACE_TPB, GRID_CAP), FACE_TPB, 0, s>>>(ca, nd, nullptr, c0, nullptr, n_faces, 0, 0,
+                                                                                          Active{nullptr, nullptr});
 }
 
 }  // namespace crush
