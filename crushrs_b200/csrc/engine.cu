@@ -539,6 +539,7 @@ struct crush_ctx {
     MaterialF32* mats = nullptr;
     Control* ctls = nullptr;      // the run, one per slot
     Control* ctls_aux = nullptr;  // drop-in calls, one per slot
+    int* slot_flags = nullptr;    // whether a resident launch gave up, then slot_done: read back in one copy
     int* slot_done = nullptr;     // per slot: done flag mirrored by the step-end kernel
     ActiveBuild ab{};             // active chunk lists of the run
     bool lists_built = false;     // they hold every running slot's chunks (a lone crash's resident steps need none)
@@ -1702,7 +1703,8 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         TRY(c->alloc(&c->sc_corner, (size_t)24 * QC));
         TRY(c->alloc(&c->ctls, cap.slots));
         TRY(c->alloc(&c->ctls_aux, cap.slots));
-        TRY(c->alloc(&c->slot_done, cap.slots));
+        TRY(c->alloc(&c->slot_flags, cap.slots + 1));
+        c->slot_done = c->slot_flags + 1;
         TRY(c->alloc(&c->mass_flag, 1));
         TRY(c->alloc(&c->fused_counter, 1));
         TRY(c->alloc(&c->forces_queue, 2));
@@ -1713,7 +1715,7 @@ int add_slots(crush_ctx* c, const crush_model_desc* const* descs, int n_desc, bo
         CK(cudaMemsetAsync(c->planes, 0, sizeof(float4) * N_STATIC_PLANES * c->stride, c->stream));
         CK(cudaMemsetAsync(c->eroded_all, 0, EC, c->stream));
         CK(cudaMemsetAsync(c->ctls, 0, sizeof(Control) * cap.slots, c->stream));
-        CK(cudaMemsetAsync(c->slot_done, 0, sizeof(int) * cap.slots, c->stream));
+        CK(cudaMemsetAsync(c->slot_flags, 0, sizeof(int) * (cap.slots + 1), c->stream));
         // contacts
         const long long KC = std::max<long long>(cap.contacts, 1), FC = std::max<long long>(cap.faces, 1),
                         SC = std::max<long long>(cap.slaves, 1), CNC = std::max<long long>(cap.cnodes, 1);
@@ -2716,6 +2718,7 @@ int run_begin(crush_ctx* c) {
     c->contact_done = false;
     c->res_unread = false;
     CK(cudaMemsetAsync(c->res_sync, 0, sizeof(ResidentSync), c->stream));
+    CK(cudaMemsetAsync(c->slot_flags, 0, sizeof(int), c->stream));
     c->lists_built = false;
     if (c->n_contacts > 0) {
         CK(cudaMemsetAsync(c->ca.big_best, 0x7F, sizeof(int) * std::max<long long>(c->n_slaves, 1), c->stream));  // BIG_NONE
@@ -3033,6 +3036,7 @@ int resident_steps(crush_ctx* c, long long n) {
     a.ctls = c->ctls;
     a.node_cn = c->node_cn;
     a.done_out = c->slot_done;
+    a.failed = c->slot_flags;
     a.mass_flag = c->mass_flag;
     a.sync = c->res_sync;
     a.step0 = c->host_step;
@@ -3127,25 +3131,30 @@ int issue_steps(crush_ctx* c, long long n_steps) {
 // Whether the resident steps issued so far went through (synchronises when
 // some were issued since the last look): a run that gave up has no state or
 // results to read, until it begins anew.
-int resident_outcome(crush_ctx* c) {
-    if (!c->res_unread) return CRUSH_OK;
-    int error = 0;
-    CK(cudaMemcpyAsync(&error, &c->res_sync->error, sizeof(error), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (error) return crush::fail(CRUSH_ERR_TIMEOUT, "a block of the resident step kernel gave up waiting at its barrier");
+int resident_outcome(crush_ctx* c, int failed) {
+    if (failed) return crush::fail(CRUSH_ERR_TIMEOUT, "a block of the resident step kernel gave up waiting at its barrier");
     c->res_unread = false;
     return CRUSH_OK;
+}
+int resident_outcome(crush_ctx* c) {
+    if (!c->res_unread) return CRUSH_OK;
+    int failed = 0;
+    CK(cudaMemcpyAsync(&failed, c->slot_flags, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return resident_outcome(c, failed);
 }
 
 // Whether every slot has finished (device flags read back; synchronises).
 int all_done(crush_ctx* c, int* done) {
-    c->done_h.resize(c->n_slots);
+    std::vector<int> flags(c->n_slots + 1);
     {
+        // the steps waited for are at work all the while
         GraphWorkScope work(c->device, c, c->run_open && !resident_fits(c));
-        CK(cudaMemcpyAsync(c->done_h.data(), c->slot_done, sizeof(int) * c->n_slots, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(flags.data(), c->slot_flags, sizeof(int) * flags.size(), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
     }
-    const int st = resident_outcome(c);
+    c->done_h.assign(flags.begin() + 1, flags.end());
+    const int st = resident_outcome(c, flags[0]);
     if (st != CRUSH_OK) return st;
     int d = 1;
     for (int x : c->done_h) d &= x ? 1 : 0;

@@ -2391,7 +2391,7 @@ cudaError_t launch_resident(cudaStream_t s, const ResidentArgs& a, int blocks) {
         if (e != cudaSuccess) return e;
     }
     const cudaError_t e = cudaLaunchCooperativeKernel(kernel, grid, tpb, args, smem, s);
-    if (e == cudaSuccess) k_steps_failed<<<(unsigned)blocks, TPB, 0, s>>>(a.sync, a.ca[0], a.n_slaves);
+    if (e == cudaSuccess) k_steps_failed<<<(unsigned)blocks, TPB, 0, s>>>(a.sync, a.failed, a.ca[0], a.n_slaves);
     return e;
 }
 void launch_node_cn(cudaStream_t s, const uint32_t* cnode, long long i0, long long i1, uint32_t* node_cn) {

@@ -424,7 +424,7 @@ void launch_frames(cudaStream_t s, const FrameArrays& f, const double* u, const 
 // ---- Resident step kernel (resident.cuh) ----
 struct ResidentSync {
     unsigned count, gen;  // grid barrier: arrivals, barriers with a serial part passed (cleared for every launch)
-    int error;            // a block gave up waiting at a barrier (cleared when a run begins, as the next)
+    int error;            // a block gave up waiting at a barrier (cleared when a run begins, as dead and ResidentArgs::failed)
     int dead;             // a launch before this one gave up
 };
 constexpr int RESIDENT_POLLS = 1 << 22;   // of a barrier before a block gives up (about 3 s), unless the caller sets another limit
@@ -439,6 +439,7 @@ struct ResidentArgs {
     Control* ctls;
     const uint32_t* node_cn;  // per node: its contact node, or CN_NONE
     int* done_out;
+    int* failed;          // what the host reads of sync->error
     int* mass_flag;
     ResidentSync* sync;
     long long step0;

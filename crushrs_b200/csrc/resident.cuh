@@ -740,9 +740,10 @@ __global__ void __launch_bounds__(RES_TPB, 1) k_steps(const __grid_constant__ Re
 // a contact search expects clear, which its half-done phase may have left set
 // (grid counts, event lists, big-face hits); the run's later launches then
 // return at once.
-__global__ void k_steps_failed(ResidentSync* y, ContactArrays ca, long long n_slaves) {
+__global__ void k_steps_failed(ResidentSync* y, int* failed, ContactArrays ca, long long n_slaves) {
     if (!y->error) return;
     y->dead = 1;
+    *failed = 1;
     const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, n = (long long)gridDim.x * blockDim.x;
     if (ca.n_contacts == 0) return;
     for (long long i = i0; i < ca.n_buckets; i += n) ca.counts[i] = 0;
