@@ -35,9 +35,10 @@
  *   - A small context's steps run in launches that hold the whole device, up
  *     to 250 steps each (4 to 20 ms). Kernels of other streams wait for a
  *     launch's end, and several small contexts take turns (which is faster
- *     than their step graphs side by side). While a context that is too large
- *     for those launches is at work on the device, the small ones step by
- *     graphs beside it; crush_set_tuning keeps a context on them.
+ *     than their step graphs side by side). While a context that does not
+ *     step so (too large, a fixed schedule, frames) is at work on the device,
+ *     the small ones step by graphs beside it; crush_set_tuning keeps a
+ *     context on them.
  */
 #ifndef CRUSH_H
 #define CRUSH_H

@@ -32,24 +32,33 @@ def _launches(ctx, steps):
     return ctx.launches() - before
 
 
+def _graphs_beside(ctx, big, steps):
+    """Whether ctx takes `steps` steps by graphs right behind an issue of the
+    large context's (which counts as at work for 5 ms from then on, so a host
+    that is slower in between tries again); the steps taken."""
+    for k in range(1, 6):
+        check(lib().crush_run_issue(big.h, 20))
+        if _launches(ctx, steps) > 100:
+            return k * steps
+    raise AssertionError("stayed resident beside the large context")
+
+
 def test_changes_over_and_back():
     small, large = _crash(0.2, 4), _crash(0.04, 28, max_steps=400)  # 384 and 131,712 elements
     alone, ctx, big = Context(small.desc), Context(small.desc), Context(large.desc)
     for c in (alone, ctx, big):
         c.run_begin()
     time.sleep(0.05)
-    alone.run_steps(200)
     assert _launches(ctx, 40) < 10  # the large context is idle
-    check(lib().crush_run_issue(big.h, 100))
-    assert _launches(ctx, 40) > 100
-    check(lib().crush_run_issue(big.h, 20))
-    assert _launches(ctx, 27) > 100
+    steps = 40 + _graphs_beside(ctx, big, 40)
+    steps += _graphs_beside(ctx, big, 27)
     big.run_steps(0)
     time.sleep(0.05)
     assert _launches(ctx, 33) < 10
     check(lib().crush_run_issue(big.h, 100))
     big.close()
     assert _launches(ctx, 60) < 10
+    alone.run_steps(steps + 93)
     assert _outcome(ctx) == _outcome(alone)
     for x, y in zip(ctx.state(), alone.state()):
         assert np.array_equal(x, y)
